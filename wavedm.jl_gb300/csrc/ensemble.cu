@@ -10,11 +10,12 @@
 // barrier whose waits are bounded: a CTA that has waited WAIT_LIMIT_NS (or
 // WAIT_MAX_POLLS polls) records WDM_DEVERR_BARRIER, raises the abort word and
 // leaves, and every other CTA leaves at its next barrier, so the launch always
-// ends.  Members keep their buffers; the pass bodies are those of the direct
-// x passes and of the line passes (xw_kick_units, xw_inv_rho_units, and
-// lfft_pipe_run, which prefetches tiles by cp.async), all with the arithmetic of
-// the per-pass launches, so a step equals those launches bit for bit.
+// ends.  Members keep their buffers; the pass bodies are those of the row
+// passes and of the register-tile line passes (kick_units, rho_units,
+// line_tile), so a step equals those launches bit for bit.
 #include "ensemble.cuh"
+#include "factor_lines.cuh"
+#include "factor_rows.cuh"
 
 #include <algorithm>
 
@@ -75,59 +76,63 @@ __device__ bool ens_grid_sync(unsigned* words, unsigned epoch, int* err) {
 // ---------------------------------------------------------------------------
 template <int N>
 constexpr size_t x_smem() {
-  return sizeof(float2) * (2 * (size_t)N + (size_t)ENS_WARPS * XCfg<N>::GROUPS * XCfg<N>::NP);
+  return fx::Rows<N>::smem(ENS_WARPS);
 }
 
-template <int N, int NTAB>
+template <int N>
 constexpr size_t line_smem() {
-  return sizeof(float2) * (2 * (size_t)NTAB * N + (size_t)(ENS_THREADS / threads_for<N>()) * 2 * N * LBUF);
+  return sizeof(float2) * (2 * (size_t)N + (size_t)(ENS_THREADS / fx::line_threads<N>()) * N * LINES);
+}
+
+template <int N>
+__device__ __forceinline__ void set_warp(fx::Warp<N>& w, const EnsMember& m, unsigned char* sm, int vb, int vg) {
+  float4* tw = reinterpret_cast<float4*>(sm);
+  load_twiddles(tw, m.twx, N);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5;
+  w.set(tw, reinterpret_cast<float2*>(sm) + 2 * N + (size_t)warp * fx::Rows<N>::WORDS,
+        XWork{m.rows.nrows / 2, m.batch}, vb * ENS_WARPS + warp, vg * ENS_WARPS);
 }
 
 template <int N, bool FWD>
 __device__ __noinline__ void x_kick(const EnsMember& m, const KickArgs& a, unsigned char* sm, int vb, int vg) {
-  using C = XCfg<N>;
-  float4* tw = reinterpret_cast<float4*>(sm);
-  load_twiddles(tw, m.twx + TW_X_FWD * N, N);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) / C::T;
-  float2* buf = reinterpret_cast<float2*>(sm) + 2 * N + (size_t)(warp * C::GROUPS + g) * C::NP;
-  const XWork w{m.rows.nrows / 2, m.batch};
-  const XSlice sl{(long long)vb * ENS_WARPS + warp, (long long)vg * ENS_WARPS, tw, buf};
-  xw_kick_units<N, FWD>(m.psi, m.psi, m.H, m.rows, m.hpitch, m.nhalf, a, w, sl);
+  fx::Warp<N> w;
+  set_warp(w, m, sm, vb, vg);
+  fx::kick_units<N, FWD>(w, m.psi, m.psi, m.H, m.rows, m.hpitch, m.nhalf, a);
   __syncthreads();
 }
 
 template <int N>
 __device__ __noinline__ void x_rho(const EnsMember& m, unsigned char* sm, int vb, int vg) {
-  using C = XCfg<N>;
-  float4* tw = reinterpret_cast<float4*>(sm);
-  load_twiddles(tw, m.twx + TW_X_FWD * N, N);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) / C::T;
-  float2* buf = reinterpret_cast<float2*>(sm) + 2 * N + (size_t)(warp * C::GROUPS + g) * C::NP;
-  const XWork w{m.rows.nrows / 2, m.batch};
-  const XSlice sl{(long long)vb * ENS_WARPS + warp, (long long)vg * ENS_WARPS, tw, buf};
-  if (m.rho.centre) xw_inv_rho_units<N, true>(m.psi, m.H, m.rows, m.hpitch, m.nhalf, m.rho, w, sl);
-  else xw_inv_rho_units<N, false>(m.psi, m.H, m.rows, m.hpitch, m.nhalf, m.rho, w, sl);
+  fx::Warp<N> w;
+  set_warp(w, m, sm, vb, vg);
+  if (m.rho.centre) fx::rho_units<N, true>(w, m.psi, m.H, m.rows, m.hpitch, m.nhalf, m.rho);
+  else fx::rho_units<N, false>(w, m.psi, m.H, m.rows, m.hpitch, m.nhalf, m.rho);
   __syncthreads();
 }
 
-// Line pass: the CTA's threads form SUB groups of threads_for<N>() that take
-// SUB consecutive tiles per round, each group prefetching its next tile by
-// cp.async into its own double buffer (lfft_pipe_run; all groups reach the
-// same barriers).
+// Line pass: the CTA's threads form SUB groups of line_threads<N>() that take
+// SUB consecutive tiles per round (line_tile; all groups reach the same
+// barriers, a group without a tile in a round works on no line).
 template <int N, int MODE, class Op>
 __device__ __noinline__ void lines(float2* data, const LineGeom& g, const float4* twg, const Op& op, int batch,
                                    unsigned char* sm, int vb, int vg) {
-  constexpr int NTAB = MODE == 2 ? 2 : 1;
-  constexpr int NT = threads_for<N>();
+  constexpr int NT = fx::line_threads<N>();
   constexpr int SUB = ENS_THREADS / NT;
   static_assert(SUB * NT == ENS_THREADS, "tile groups fill the CTA");
   float4* tw = reinterpret_cast<float4*>(sm);
-  load_twiddles(tw, twg + TW_LINE_FWD * N, NTAB * N);  // visible after the first round's barrier
+  load_twiddles(tw, twg, N);  // visible after the first round's barrier
   const int sub = threadIdx.x / NT, tid = threadIdx.x % NT;
-  float2* bufs = reinterpret_cast<float2*>(sm) + 2 * NTAB * N + (size_t)sub * 2 * N * LBUF;
-  lfft_pipe_run<N, MODE, Op>(data, g, tw, op, batch, bufs, tid, (long long)vb * SUB, (long long)vg * SUB, sub);
+  float2* buf = reinterpret_cast<float2*>(sm) + 2 * N + (size_t)sub * N * LINES;
+  const int tiles = (g.nlines + LINES - 1) / LINES;
+  const long long total = (long long)tiles * batch;
+  for (long long base = (long long)vb * SUB; base < total; base += (long long)vg * SUB) {
+    const long long tile = base + sub;
+    const int b = tile < total ? (int)(tile / tiles) : 0;
+    const int line0 = tile < total ? (int)(tile - (long long)b * tiles) * LINES : g.nlines;
+    fx::line_tile<N, MODE, Op>(data, g, tw, op, line0, b, buf, tid);
+    __syncthreads();  // the buffer is read before the next round fills it
+  }
   __syncthreads();
 }
 
@@ -183,13 +188,13 @@ __device__ void member_pass(const EnsMember& m, int p, int s, int mode, unsigned
       pass_x_kick(m, full ? m.kick_full : m.kick_half, true, sm, vb, vg);
       break;
     }
-    case 1: pass_lines<0>(m.ny, m.psi, m.ly_psi, m.twy, NoOp{}, m.batch, sm, vb, vg); break;
-    case 2: pass_lines<2>(m.nz, m.psi, m.lz_psi, m.twz, m.drift, m.batch, sm, vb, vg); break;
-    case 3: pass_lines<1>(m.ny, m.psi, m.ly_psi, m.twy, NoOp{}, m.batch, sm, vb, vg); break;
+    case 1: pass_lines<0>(m.ny, m.psi, m.ly_psi, m.twy, fx::None{}, m.batch, sm, vb, vg); break;
+    case 2: pass_lines<2>(m.nz, m.psi, m.lz_psi, m.twz, fx::Drift{m.drift}, m.batch, sm, vb, vg); break;
+    case 3: pass_lines<1>(m.ny, m.psi, m.ly_psi, m.twy, fx::None{}, m.batch, sm, vb, vg); break;
     case 4: pass_x_rho(m, sm, vb, vg); break;
-    case 5: pass_lines<0>(m.ny, m.H, m.ly_h, m.twy, NoOp{}, m.batch, sm, vb, vg); break;
-    case 6: pass_lines<2>(m.nz, m.H, m.lz_h, m.twz, m.poisson, m.batch, sm, vb, vg); break;
-    case 7: pass_lines<1>(m.ny, m.H, m.ly_h, m.twy, NoOp{}, m.batch, sm, vb, vg); break;
+    case 5: pass_lines<0>(m.ny, m.H, m.ly_h, m.twy, fx::None{}, m.batch, sm, vb, vg); break;
+    case 6: pass_lines<2>(m.nz, m.H, m.lz_h, m.twz, fx::Poisson{m.poisson}, m.batch, sm, vb, vg); break;
+    case 7: pass_lines<1>(m.ny, m.H, m.ly_h, m.twy, fx::None{}, m.batch, sm, vb, vg); break;
     default: pass_x_kick(m, m.kick_half, false, sm, vb, vg); break;
   }
 }
@@ -220,10 +225,10 @@ k_ensemble(const EnsMember* __restrict__ mem, int nmem, int nsteps, int mode, un
     for (int m = 0; m < nmem; ++m) member_pass(mem[m], 8, nsteps, mode, esm, (blockIdx.x + mem[m].rot) % vg, vg);
 }
 
-size_t smem_for_axis(int n, int kind) {  // kind 0: x pass, 1: y lines, 2: z lines (two tables)
+size_t smem_for_axis(int n, int kind) {  // kind 0: x pass, else lines
   switch (n) {
 #define WDM_CASE(N_) \
-  case N_: return kind == 0 ? x_smem<N_>() : (kind == 1 ? line_smem<N_, 1>() : line_smem<N_, 2>());
+  case N_: return kind == 0 ? x_smem<N_>() : line_smem<N_>();
     WDM_ENS_SIZES(WDM_CASE)
 #undef WDM_CASE
   }

@@ -8,10 +8,9 @@
 namespace wdm {
 
 // One member context as the persistent kernel sees it (filled on the host,
-// kept in device memory).  The kernel runs the pass bodies of the direct x
-// passes and the register-tile line passes, the same arithmetic as those
-// launches, so its results equal the per-pass launches of that schedule bit
-// for bit.
+// kept in device memory).  The kernel runs the pass bodies of the row passes and
+// of the register-tile line passes, so its results equal the per-pass launches
+// bit for bit.
 struct EnsMember {
   int nx, ny, nz, batch;
   float2* psi;

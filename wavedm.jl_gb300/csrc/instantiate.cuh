@@ -1,118 +1,13 @@
 // Launchers of the pass kernels for one axis length N (included by sizes_*.cu).
 #pragma once
-#include <atomic>
-#include <cmath>
-#include "kernel_set.h"
+#include "launch_util.cuh"
 #include "xpass_warp.cuh"
 
 namespace wdm {
 
-// Launch settings are device properties: each is found once per device (the
-// current one at the launch) and kept in a slot per device ordinal.
-constexpr int MAX_DEVICES = 64;
-
-static int current_device() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  return dev >= 0 && dev < MAX_DEVICES ? dev : 0;
-}
-
-// Opt a kernel in to more than 48 KB of dynamic shared memory, once per device.
-template <auto K>
-static cudaError_t prep_once(size_t smem) {
-  if (smem <= 48 * 1024) return cudaSuccess;
-  // 0: not yet, 1: done, 2 + e: failed with cudaError_t e
-  static std::atomic<int> state[MAX_DEVICES];
-  std::atomic<int>& st = state[current_device()];
-  int v = st.load(std::memory_order_acquire);
-  if (v == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    v = e == cudaSuccess ? 1 : 2 + (int)e;
-    st.store(v, std::memory_order_release);
-  }
-  return v == 1 ? cudaSuccess : (cudaError_t)(v - 2);
-}
-
-// SMs of the current device.
-static int sm_count() {
-  static std::atomic<int> n[MAX_DEVICES];
-  const int dev = current_device();
-  int v = n[dev].load(std::memory_order_relaxed);
-  if (v == 0) {
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    v = v > 0 ? v : 1;
-    n[dev].store(v, std::memory_order_relaxed);
-  }
-  return v;
-}
-
-// Resident CTAs per SM of a kernel at its block size and shared memory, on the
-// current device (each call site passes one fixed size).
-template <auto K>
-static int resident_ctas(int threads, size_t smem) {
-  static std::atomic<int> n[MAX_DEVICES];
-  std::atomic<int>& slot = n[current_device()];
-  int v = slot.load(std::memory_order_relaxed);
-  if (v == 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, K, threads, smem);
-    v = v > 0 ? v : 1;
-    slot.store(v, std::memory_order_relaxed);
-  }
-  return v;
-}
-
 template <int N>
 struct Launch {
   static constexpr int NT = threads_for<N>();
-
-  // Tensor map of the lines of g (null view: false).
-  static bool line_map(CUtensorMap* map, const float2* data, const LineGeom& g, int batch) {
-    using TT = TmaTile<N>;
-    if (g.axis != 1 && g.axis != 2) return false;
-    if (g.nxa < LINES || g.rows <= 0) return false;  // the box stays inside the tensor along x
-    const uint64_t e = sizeof(float2);
-    uint64_t dims[4], strides[3];
-    uint32_t box[4];
-    dims[0] = (uint64_t)g.nxa;
-    dims[3] = (uint64_t)batch;
-    strides[0] = (uint64_t)g.pitch * e;
-    strides[2] = (uint64_t)g.bstride * e;
-    if (g.axis == 1) {  // [batch][rows][N][pitch]
-      dims[1] = N;
-      dims[2] = (uint64_t)g.rows;
-      strides[1] = (uint64_t)g.pitch * N * e;
-      box[0] = LINES, box[1] = TT::BOXP, box[2] = 1, box[3] = 1;
-    } else {  // [batch][N][rows][pitch]
-      dims[1] = (uint64_t)g.rows;
-      dims[2] = N;
-      strides[1] = (uint64_t)g.pitch * g.rows * e;
-      box[0] = LINES, box[1] = 1, box[2] = TT::BOXP, box[3] = 1;
-    }
-    return encode_map_c64(map, data, dims, strides, box);
-  }
-
-  // Tensor map of the edge tiles of g (the last column when nxa = 16 m + 1,
-  // 8 rows per tile; k_lfft_tma): the lines' axis outermost, a box of 2
-  // columns x 8 rows x BOXP points starting at column nxa - 1, whose x offset
-  // (nxa - 1) * 8 bytes must be a multiple of 16.  false: no edge tiles.
-  static bool edge_map(CUtensorMap* map, const float2* data, const LineGeom& g, int batch) {
-    using TT = TmaTile<N>;
-    if (g.axis != 1 && g.axis != 2) return false;
-    if (g.nxa % LINES != 1 || g.nxa < LINES || (g.nxa - 1) % 2 != 0 || g.rows <= 0 || g.rows % 8 != 0) return false;
-    const uint64_t e = sizeof(float2);
-    uint64_t dims[4] = {(uint64_t)g.nxa, (uint64_t)g.rows, (uint64_t)N, (uint64_t)batch};
-    uint64_t strides[3];
-    if (g.axis == 1) {  // rows (z) at pitch * N, points (y) at pitch
-      strides[0] = (uint64_t)g.pitch * N * e;
-      strides[1] = (uint64_t)g.pitch * e;
-    } else {  // rows (y) at pitch, points (z) at pitch * rows
-      strides[0] = (uint64_t)g.pitch * e;
-      strides[1] = (uint64_t)g.pitch * g.rows * e;
-    }
-    strides[2] = (uint64_t)g.bstride * e;
-    const uint32_t box[4] = {2, 8, (uint32_t)TT::BOXP, 1};
-    return encode_map_c64(map, data, dims, strides, box);
-  }
 
   template <int MODE, bool LATE, class Op>
   static cudaError_t ltma_launch(float2* data, const CUtensorMap& map, const CUtensorMap& emap, const LineGeom& ge,
@@ -137,11 +32,11 @@ struct Launch {
 #if !defined(WDM_LINE_PIPELINE) && !defined(WDM_LINE_TILE)
     {
       CUtensorMap map, emap;
-      if (g.impl == LINE_IMPL_TMA && line_map(&map, data, g, batch)) {
+      if (g.impl == LINE_IMPL_TMA && LineMaps<N>::line_map(&map, data, g, batch)) {
         LineGeom ge = g;
         ge.edge = 0;
 #ifndef WDM_NO_EDGE_TILES
-        if (edge_map(&emap, data, g, batch)) ge.edge = g.rows / 8;
+        if (LineMaps<N>::edge_map(&emap, data, g, batch)) ge.edge = g.rows / 8;
 #endif
         if (!ge.edge) emap = map;  // not read
         // The next tile's copy goes out late (k_lfft_tma) in the fused z

@@ -16,6 +16,7 @@
 #include "../../include/wavedm.h"
 #include "aux_kernels.cuh"
 #include "ensemble.cuh"
+#include "factor_set.h"
 #include "kernel_set.h"
 
 namespace wdm {
@@ -50,6 +51,39 @@ const KernelSet* kernels_for(int n) {
     case 256: return ks_256();
     case 384: return ks_384();
     case 512: return ks_512();
+    default: return nullptr;
+  }
+}
+
+const FactorSet* fs_8();
+const FactorSet* fs_12();
+const FactorSet* fs_16();
+const FactorSet* fs_24();
+const FactorSet* fs_32();
+const FactorSet* fs_48();
+const FactorSet* fs_64();
+const FactorSet* fs_96();
+const FactorSet* fs_128();
+const FactorSet* fs_192();
+const FactorSet* fs_256();
+const FactorSet* fs_384();
+const FactorSet* fs_512();
+
+const FactorSet* factors_for(int n) {
+  switch (n) {
+    case 8: return fs_8();
+    case 12: return fs_12();
+    case 16: return fs_16();
+    case 24: return fs_24();
+    case 32: return fs_32();
+    case 48: return fs_48();
+    case 64: return fs_64();
+    case 96: return fs_96();
+    case 128: return fs_128();
+    case 192: return fs_192();
+    case 256: return fs_256();
+    case 384: return fs_384();
+    case 512: return fs_512();
     default: return nullptr;
   }
 }
@@ -115,7 +149,13 @@ struct wdm_ctx {
   long long ncell = 0;   // cells per batch item
   long long nhalf = 0;   // H entries per batch item (hpitch * ny * nz, the batch stride)
   cudaStream_t st = nullptr;
+  // the two-factor passes of the axes (time step, Poisson solve, plain
+  // transforms) and their twiddles; kx, ky, kz and twx, twy, twz: the Stockham
+  // passes, which the adjoint runs on (fft_factor.cuh says why)
+  const FactorSet *fx = nullptr, *fy = nullptr, *fz = nullptr;
+  float4 *ftx = nullptr, *fty = nullptr, *ftz = nullptr;
   const KernelSet *kx = nullptr, *ky = nullptr, *kz = nullptr;
+  int stockham = 0;  // set while the adjoint runs
   double dx = 0, dy = 0, dz = 0, x0 = 0, y0 = 0, z0 = 0;
   // device buffers
   float2* psi = nullptr;
@@ -157,6 +197,9 @@ struct wdm_ctx {
   int64_t launch_count = 0;
   // autotuned implementation of each line pass (LP_*) and the candidate timings
   int line_impl[LP_COUNT] = {0, 0, 0, 0, 0, 0, 0};
+  // the same of the adjoint's Stockham passes, found at the first adjoint
+  int adj_impl[LP_COUNT] = {0, 0, 0, 0, 0, 0, 0};
+  double adj_ms[LP_COUNT][2] = {};
   double line_ms[LP_COUNT][2] = {{-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}};
   // adjoint buffers (allocated on first use)
   float2* lam = nullptr;            // adjoint state [batch][ncell]
@@ -353,6 +396,14 @@ static wdm_status upload_twiddles(wdm_ctx* c, float4** dst, const KernelSet* ks)
   return WDM_OK;
 }
 
+static wdm_status upload_factors(wdm_ctx* c, float4** dst, const FactorSet* fs) {
+  std::vector<float4> h((size_t)fs->n);
+  fs->fill_twiddles(h.data());
+  WDM_TRY(dalloc(c, dst, h.size()));
+  WDM_CU(c, cudaMemcpy(*dst, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
+  return WDM_OK;
+}
+
 static wdm_status upload_k2(wdm_ctx* c, float** dst, int n, double L) {
   std::vector<float> h(n);
   for (int m = 0; m < n; ++m) {
@@ -425,6 +476,10 @@ static wdm_status ensure_mask_tables(wdm_ctx* c, double dt) {
   return WDM_OK;
 }
 
+// The implementations of the passes the context is running on.
+static int* impls(wdm_ctx* c) { return c->stockham ? c->adj_impl : c->line_impl; }
+static const int* impls(const wdm_ctx* c) { return c->stockham ? c->adj_impl : c->line_impl; }
+
 static RowGeom rows_psi(const wdm_ctx* c) {
   RowGeom r;
   r.nrows = c->d.ny * c->d.nz;
@@ -437,7 +492,7 @@ static RowGeom rows_psi(const wdm_ctx* c) {
 // The rows of psi for the tuned x pass `kind` (LP_X_KICK, LP_X_RHO or LP_X_RHO_B).
 static RowGeom rows_psi(const wdm_ctx* c, int kind) {
   RowGeom r = rows_psi(c);
-  r.impl = c->line_impl[kind];
+  r.impl = impls(c)[kind];
   return r;
 }
 
@@ -454,7 +509,7 @@ static LineGeom lines_y(const wdm_ctx* c, int xext, long long pitch, long long b
   g.rows = c->d.nz;
   g.pitch = pitch;
   g.err = c->flag + 1;
-  g.impl = c->line_impl[xext == c->nxh ? LP_H_Y : LP_PSI_Y];
+  g.impl = impls(c)[xext == c->nxh ? LP_H_Y : LP_PSI_Y];
   return g;
 }
 
@@ -469,13 +524,37 @@ static LineGeom lines_z(const wdm_ctx* c, int xext, long long pitch, long long b
   g.rows = c->d.ny;
   g.pitch = pitch;
   g.err = c->flag + 1;
-  g.impl = c->line_impl[xext == c->nxh ? LP_H_Z : LP_PSI_Z];
+  g.impl = impls(c)[xext == c->nxh ? LP_H_Z : LP_PSI_Z];
   return g;
 }
 
 // --------------------------------------------------------------------------
 // pipeline pieces
 // --------------------------------------------------------------------------
+// One pass on the kernels the context is running on: the two-factor passes, or
+// the Stockham passes while the adjoint runs.
+static cudaError_t y_lines(wdm_ctx* c, float2* data, const LineGeom& g, bool inv) {
+  return c->stockham ? c->ky->lfft(data, g, c->twy, inv, c->d.batch, c->st)
+                     : c->fy->line(data, g, c->fty, inv, c->d.batch, c->st);
+}
+static cudaError_t z_drift(wdm_ctx* c, float2* data, const LineGeom& g, const DriftOp& op) {
+  return c->stockham ? c->kz->lfft_drift(data, g, c->twz, op, c->d.batch, c->st)
+                     : c->fz->line_drift(data, g, c->ftz, op, c->d.batch, c->st);
+}
+static cudaError_t z_poisson(wdm_ctx* c, float2* data, const LineGeom& g, const PoissonOp& op) {
+  return c->stockham ? c->kz->lfft_poisson(data, g, c->twz, op, c->d.batch, c->st)
+                     : c->fz->line_poisson(data, g, c->ftz, op, c->d.batch, c->st);
+}
+static cudaError_t x_rho(wdm_ctx* c, const RhoArgs& a, int kind) {
+  return c->stockham ? c->kx->x_inv_rho(c->psi, c->H, rows_psi(c, kind), c->hpitch, c->nhalf, c->twx, a, c->d.batch, c->st)
+                     : c->fx->rho(c->psi, c->H, rows_psi(c), c->hpitch, c->nhalf, c->ftx, a, c->d.batch, c->st);
+}
+static cudaError_t x_kick(wdm_ctx* c, const float2* in, const KickArgs& a, bool fwd) {
+  return c->stockham ? c->kx->x_kick(in, c->psi, c->H, rows_psi(c, LP_X_KICK), c->hpitch, c->nhalf, c->twx, a, fwd,
+                                     c->d.batch, c->st)
+                     : c->fx->kick(in, c->psi, c->H, rows_psi(c), c->hpitch, c->nhalf, c->ftx, a, fwd, c->d.batch, c->st);
+}
+
 // density (+baryons) of psi -> H, then the Poisson solve on H (P5..P8).
 // The CIC deposit of the current particles into rho_b (zero before it), made
 // once per particle set.
@@ -514,11 +593,10 @@ static wdm_status density_poisson(wdm_ctx* c, int write_psi, double dt_mask) {
     ra.centre = c->centre;
   }
   cudaError_t e = run_pass(c, write_psi ? P_X_INV_RHO : P_DENSITY, [&] {
-    return c->kx->x_inv_rho(c->psi, c->H, rows_psi(c, c->nparts > 0 ? LP_X_RHO_B : LP_X_RHO), c->hpitch, c->nhalf,
-                            c->twx, ra, B, c->st);
+    return x_rho(c, ra, c->nparts > 0 ? LP_X_RHO_B : LP_X_RHO);
   });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_inv_rho");
-  if ((e = run_pass(c, P_H_Y_FWD, [&] { return c->ky->lfft(c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), c->twy, false, B, c->st); })) !=
+  if ((e = run_pass(c, P_H_Y_FWD, [&] { return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), false); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "H y fwd");
   PoissonOp po;
@@ -527,10 +605,10 @@ static wdm_status density_poisson(wdm_ctx* c, int write_psi, double dt_mask) {
   po.kz2 = c->kz2;
   po.coef = (float)(-c->d.poisson_coeff / ((double)c->d.nx * c->d.ny * c->d.nz));
   if ((e = run_pass(c, P_H_Z_POISSON,
-                    [&] { return c->kz->lfft_poisson(c->H, lines_z(c, c->nxh, c->hpitch, c->nhalf), c->twz, po, B, c->st); })) !=
+                    [&] { return z_poisson(c, c->H, lines_z(c, c->nxh, c->hpitch, c->nhalf), po); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "H z poisson");
-  if ((e = run_pass(c, P_H_Y_INV, [&] { return c->ky->lfft(c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), c->twy, true, B, c->st); })) !=
+  if ((e = run_pass(c, P_H_Y_INV, [&] { return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), true); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "H y inv");
   c->phi_valid = 1;
@@ -613,7 +691,7 @@ static wdm_status kick(wdm_ctx* c, double dt, int sched_row, bool fwd, const flo
   }
   const float2* in = psi_in ? psi_in : c->psi;
   cudaError_t e = run_pass(c, fwd ? P_KICK_FWD : P_KICK, [&] {
-    return c->kx->x_kick(in, c->psi, c->H, rows_psi(c, LP_X_KICK), c->hpitch, c->nhalf, c->twx, a, fwd, c->d.batch, c->st);
+    return x_kick(c, in, a, fwd);
   });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_kick");
   return WDM_OK;
@@ -623,7 +701,6 @@ static wdm_status kick(wdm_ctx* c, double dt, int sched_row, bool fwd, const flo
 // phase * inverse, y inverse.  sign = -1 applies the conjugate phase (the
 // drift adjoint).
 static wdm_status drift_yz(wdm_ctx* c, double dt, float sign = 1.f, float2* data = nullptr) {
-  const int B = c->d.batch;
   float2* psi = data ? data : c->psi;
   DriftOp op{};
   op.sign = sign;
@@ -641,15 +718,15 @@ static wdm_status drift_yz(wdm_ctx* c, double dt, float sign = 1.f, float2* data
   op.precise = precise;
   cudaError_t e;
   if ((e = run_pass(c, P_PSI_Y_FWD,
-                    [&] { return c->ky->lfft(psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), c->twy, false, B, c->st); })) !=
+                    [&] { return y_lines(c, psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), false); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "psi y fwd");
   if ((e = run_pass(c, P_PSI_Z_DRIFT,
-                    [&] { return c->kz->lfft_drift(psi, lines_z(c, c->d.nx, c->d.nx, c->ncell), c->twz, op, B, c->st); })) !=
+                    [&] { return z_drift(c, psi, lines_z(c, c->d.nx, c->d.nx, c->ncell), op); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "psi z drift");
   if ((e = run_pass(c, P_PSI_Y_INV,
-                    [&] { return c->ky->lfft(psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), c->twy, true, B, c->st); })) !=
+                    [&] { return y_lines(c, psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), true); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "psi y inv");
   return WDM_OK;
@@ -728,7 +805,7 @@ wdm_status wdm_destroy(wdm_ctx* c) {
                   c->scratch_h, c->red, c->sums, c->shift, c->shift_in};
   for (void* p : bufs)
     if (p) cudaFree(p);
-  void* adj[] = {c->lam, c->Hmu, c->rho_t, c->D6, c->adj_acc, c->diag_wsum, c->diag_wmin, c->centre, c->frame};
+  void* adj[] = {c->ftx, c->fty, c->ftz, c->lam, c->Hmu, c->rho_t, c->D6, c->adj_acc, c->diag_wsum, c->diag_wmin, c->centre, c->frame};
   for (void* p : adj)
     if (p) cudaFree(p);
   for (auto* v : {&c->ck_psi, &c->ck_H, &c->slot_psi, &c->slot_H, &c->slot2_psi, &c->slot2_H})
@@ -759,8 +836,11 @@ wdm_status wdm_destroy(wdm_ctx* c) {
 // pass on its own buffers (zeroed; the fused z passes with the Poisson
 // operator, the kick with a small time step) and keeps the faster, preferring
 // implementation 0 within 3%.  Choices are kept per (device, nx, ny, nz,
-// batch); WDM_LINE_IMPL=tma|tile and WDM_X_IMPL=staged|direct force them.
-using TuneKey = std::tuple<int, int, int, int, int>;
+// batch, kernels); WDM_LINE_IMPL=tma|tile and WDM_X_IMPL=staged|direct force
+// them.  The x choices are the adjoint's alone: the row passes of the time
+// step have one implementation.  The adjoint's passes are timed at its first
+// run, on its own buffers.
+using TuneKey = std::tuple<int, int, int, int, int, int>;
 struct TuneVal {
   int impl[LP_COUNT];
   double ms[LP_COUNT][2];
@@ -772,12 +852,12 @@ static std::map<TuneKey, TuneVal> g_tune_cache;
 static void forced_impls(wdm_ctx* c) {
   if (const char* env = std::getenv("WDM_LINE_IMPL")) {
     if (!std::strcmp(env, "tma") || !std::strcmp(env, "tile"))
-      for (int k = LP_PSI_Y; k <= LP_H_Z; ++k) c->line_impl[k] = std::strcmp(env, "tma") ? LINE_IMPL_TILE : LINE_IMPL_TMA;
+      for (int k = LP_PSI_Y; k <= LP_H_Z; ++k) impls(c)[k] = std::strcmp(env, "tma") ? LINE_IMPL_TILE : LINE_IMPL_TMA;
   }
   if (const char* env = std::getenv("WDM_X_IMPL")) {
     if (!std::strcmp(env, "staged") || !std::strcmp(env, "direct"))
       for (int k = LP_X_KICK; k <= LP_X_RHO_B; ++k)
-        c->line_impl[k] = std::strcmp(env, "staged") ? X_IMPL_DIRECT : X_IMPL_STAGED;
+        impls(c)[k] = std::strcmp(env, "staged") ? X_IMPL_DIRECT : X_IMPL_STAGED;
   }
 }
 
@@ -803,7 +883,7 @@ static bool schedule_from_env(wdm_ctx* c) {
     if (end == std::string::npos && k + 1 < LP_COUNT) return false;
     pos = end + 1;
   }
-  std::memcpy(c->line_impl, impl, sizeof(impl));
+  std::memcpy(impls(c), impl, sizeof(impl));
   return true;
 }
 
@@ -814,15 +894,18 @@ static wdm_status tune_passes(wdm_ctx* c) {
   return WDM_OK;
 }
 
+// Times on psi and H, which it clears.
 static wdm_status tune_passes_timed(wdm_ctx* c) {
   int dev = 0;
   WDM_CU(c, cudaGetDevice(&dev));
-  const TuneKey key{dev, c->d.nx, c->d.ny, c->d.nz, c->d.batch};
+  int* impl = impls(c);
+  auto* times = c->stockham ? c->adj_ms : c->line_ms;
+  const TuneKey key{dev, c->d.nx, c->d.ny, c->d.nz, c->d.batch, c->stockham};
   std::lock_guard<std::mutex> lock(g_tune_mu);
   auto hit = g_tune_cache.find(key);
   if (hit != g_tune_cache.end()) {
-    std::memcpy(c->line_impl, hit->second.impl, sizeof(c->line_impl));
-    std::memcpy(c->line_ms, hit->second.ms, sizeof(c->line_ms));
+    std::memcpy(impl, hit->second.impl, sizeof(hit->second.impl));
+    std::memcpy(times, hit->second.ms, sizeof(hit->second.ms));
     return WDM_OK;
   }
   const int B = c->d.batch;
@@ -841,19 +924,17 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
   ra.err = c->flag + 1;
   auto run = [&](int k) -> cudaError_t {
     switch (k) {
-      case LP_PSI_Y: return c->ky->lfft(c->psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), c->twy, false, B, c->st);
-      case LP_PSI_Z: return c->kz->lfft_poisson(c->psi, lines_z(c, c->d.nx, c->d.nx, c->ncell), c->twz, po, B, c->st);
-      case LP_H_Y: return c->ky->lfft(c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), c->twy, false, B, c->st);
-      case LP_H_Z: return c->kz->lfft_poisson(c->H, lines_z(c, c->nxh, c->hpitch, c->nhalf), c->twz, po, B, c->st);
-      case LP_X_KICK:
-        return c->kx->x_kick(c->psi, c->psi, c->H, rows_psi(c, LP_X_KICK), c->hpitch, c->nhalf, c->twx, ka, true, B,
-                             c->st);
-      case LP_X_RHO: return c->kx->x_inv_rho(c->psi, c->H, rows_psi(c, LP_X_RHO), c->hpitch, c->nhalf, c->twx, ra, B, c->st);
+      case LP_PSI_Y: return y_lines(c, c->psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), false);
+      case LP_PSI_Z: return z_poisson(c, c->psi, lines_z(c, c->d.nx, c->d.nx, c->ncell), po);
+      case LP_H_Y: return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), false);
+      case LP_H_Z: return z_poisson(c, c->H, lines_z(c, c->nxh, c->hpitch, c->nhalf), po);
+      case LP_X_KICK: return x_kick(c, c->psi, ka, true);
+      case LP_X_RHO: return x_rho(c, ra, k);
       default: {
         // a stand-in baryon density: the zeroed psi buffer, read as floats
         RhoArgs rb = ra;
         rb.rho_b = reinterpret_cast<const float*>(c->psi);
-        return c->kx->x_inv_rho(c->psi, c->H, rows_psi(c, LP_X_RHO_B), c->hpitch, c->nhalf, c->twx, rb, B, c->st);
+        return x_rho(c, rb, k);
       }
     }
   };
@@ -862,8 +943,12 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
   WDM_CU(c, cudaEventCreate(&e1));
   cudaError_t e = cudaSuccess;
   for (int k = 0; k < LP_COUNT && e == cudaSuccess; ++k) {
-    for (int impl = 0; impl <= 1 && e == cudaSuccess; ++impl) {
-      c->line_impl[k] = impl;
+    for (int q = 0; q <= 1 && e == cudaSuccess; ++q) {
+      impl[k] = q;
+      if (q == 1 && k >= LP_X_KICK && !c->stockham) {  // the two-factor row passes have one implementation
+        times[k][1] = times[k][0];
+        break;
+      }
       double best = 1e30;
       for (int r = 0; r < 4 && e == cudaSuccess; ++r) {  // the first run is a warm-up
         if ((e = cudaEventRecord(e0, c->st)) != cudaSuccess || (e = run(k)) != cudaSuccess ||
@@ -873,16 +958,16 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
         if ((e = cudaEventElapsedTime(&ms, e0, e1)) != cudaSuccess) break;
         if (r > 0 && ms < best) best = ms;
       }
-      c->line_ms[k][impl] = best;
+      times[k][q] = best;
     }
-    c->line_impl[k] = c->line_ms[k][1] < 0.97 * c->line_ms[k][0] ? 1 : 0;
+    impl[k] = times[k][1] < 0.97 * times[k][0] ? 1 : 0;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (e != cudaSuccess) return cuda_fail(c, e, "line-pass autotuner");
   TuneVal v;
-  std::memcpy(v.impl, c->line_impl, sizeof(v.impl));
-  std::memcpy(v.ms, c->line_ms, sizeof(v.ms));
+  std::memcpy(v.impl, impl, sizeof(v.impl));
+  std::memcpy(v.ms, times, sizeof(v.ms));
   g_tune_cache[key] = v;
   return WDM_OK;
 }
@@ -924,6 +1009,9 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
   c->hpitch = (c->nxh + WDM_HPITCH_ALIGN - 1) / WDM_HPITCH_ALIGN * WDM_HPITCH_ALIGN;
 #endif
   c->nhalf = (long long)c->hpitch * d->ny * d->nz;
+  c->fx = factors_for(d->nx);
+  c->fy = factors_for(d->ny);
+  c->fz = factors_for(d->nz);
   c->kx = kernels_for(d->nx);
   c->ky = kernels_for(d->ny);
   c->kz = kernels_for(d->nz);
@@ -944,9 +1032,9 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
   const size_t B = (size_t)d->batch;
   if ((s = dalloc(c, &c->psi, B * ncell)) != WDM_OK) return bail(s);
   if ((s = dalloc(c, &c->H, B * c->nhalf)) != WDM_OK) return bail(s);
-  if ((s = upload_twiddles(c, &c->twx, c->kx)) != WDM_OK) return bail(s);
-  if ((s = upload_twiddles(c, &c->twy, c->ky)) != WDM_OK) return bail(s);
-  if ((s = upload_twiddles(c, &c->twz, c->kz)) != WDM_OK) return bail(s);
+  if ((s = upload_factors(c, &c->ftx, c->fx)) != WDM_OK) return bail(s);
+  if ((s = upload_factors(c, &c->fty, c->fy)) != WDM_OK) return bail(s);
+  if ((s = upload_factors(c, &c->ftz, c->fz)) != WDM_OK) return bail(s);
   if ((s = upload_k2(c, &c->kx2, d->nx, d->lx)) != WDM_OK) return bail(s);
   if ((s = upload_k2(c, &c->ky2, d->ny, d->ly)) != WDM_OK) return bail(s);
   if ((s = upload_k2(c, &c->kz2, d->nz, d->lz)) != WDM_OK) return bail(s);
@@ -1006,7 +1094,7 @@ static wdm_status phi_real(wdm_ctx* c) {
   WDM_TRY(ensure_scratch(c));
   if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, 0.0));
   cudaError_t e = run_pass(c, P_PHI_OUT, [&] {
-    return c->kx->x_c2r(c->H, c->scratch_f, rows_psi(c), c->hpitch, c->nhalf, c->twx, c->d.batch, c->st);
+    return c->fx->c2r(c->H, c->scratch_f, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
   });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_c2r");
   return WDM_OK;
@@ -1192,7 +1280,7 @@ wdm_status wdm_kick(wdm_ctx* c, double dt, double t) {
 
 wdm_status wdm_drift(wdm_ctx* c, double dt) {
   WDM_TRY(need_psi(c));
-  cudaError_t e = run_pass(c, P_X_FFT, [&] { return c->kx->xfft(c->psi, rows_psi(c), c->twx, false, 1.0f, c->d.batch, c->st); });
+  cudaError_t e = run_pass(c, P_X_FFT, [&] { return c->fx->fft(c->psi, rows_psi(c), c->ftx, false, 1.0f, c->d.batch, c->st); });
   if (e != cudaSuccess) return cuda_fail(c, e, "x fwd");
   WDM_TRY(drift_yz(c, dt));
   WDM_TRY(density_poisson(c, 1, dt));
@@ -1215,21 +1303,21 @@ wdm_status wdm_poisson(wdm_ctx* c, const float* rho, float* phi, int32_t where) 
   cudaError_t e;
   if ((e = launch_mean_shift(in, false, c->ncell, B, c->sums, c->shift_in, 0.0, c->st)) != cudaSuccess)
     return cuda_fail(c, e, "mean");
-  if ((e = c->kx->x_r2c(in, c->scratch_h, rows_psi(c), c->hpitch, c->nhalf, c->twx, c->shift_in, B, c->st)) != cudaSuccess)
+  if ((e = c->fx->r2c(in, c->scratch_h, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->shift_in, B, c->st)) != cudaSuccess)
     return cuda_fail(c, e, "x r2c");
-  if ((e = c->ky->lfft(c->scratch_h, lines_y(c, c->nxh, c->hpitch, c->nhalf), c->twy, false, B, c->st)) != cudaSuccess)
+  if ((e = y_lines(c, c->scratch_h, lines_y(c, c->nxh, c->hpitch, c->nhalf), false)) != cudaSuccess)
     return cuda_fail(c, e, "y fwd");
   PoissonOp po;
   po.kx2 = c->kx2;
   po.ky2 = c->ky2;
   po.kz2 = c->kz2;
   po.coef = (float)(-c->d.poisson_coeff / ((double)c->d.nx * c->d.ny * c->d.nz));
-  if ((e = c->kz->lfft_poisson(c->scratch_h, lines_z(c, c->nxh, c->hpitch, c->nhalf), c->twz, po, B, c->st)) != cudaSuccess)
+  if ((e = z_poisson(c, c->scratch_h, lines_z(c, c->nxh, c->hpitch, c->nhalf), po)) != cudaSuccess)
     return cuda_fail(c, e, "z poisson");
-  if ((e = c->ky->lfft(c->scratch_h, lines_y(c, c->nxh, c->hpitch, c->nhalf), c->twy, true, B, c->st)) != cudaSuccess)
+  if ((e = y_lines(c, c->scratch_h, lines_y(c, c->nxh, c->hpitch, c->nhalf), true)) != cudaSuccess)
     return cuda_fail(c, e, "y inv");
   float* dst = where == WDM_HOST ? c->scratch_f : phi;
-  if ((e = c->kx->x_c2r(c->scratch_h, dst, rows_psi(c), c->hpitch, c->nhalf, c->twx, B, c->st)) != cudaSuccess)
+  if ((e = c->fx->c2r(c->scratch_h, dst, rows_psi(c), c->hpitch, c->nhalf, c->ftx, B, c->st)) != cudaSuccess)
     return cuda_fail(c, e, "x c2r");
   if (where == WDM_HOST) return copy_out(c, phi, c->scratch_f, bytes, WDM_HOST);
   WDM_CU(c, cudaStreamSynchronize(c->st));
@@ -1244,10 +1332,10 @@ wdm_status wdm_fft3d(wdm_ctx* c, void* data, int32_t dir) {
   const int B = c->d.batch;
   float2* p = (float2*)data;
   cudaError_t e;
-  if ((e = c->kx->xfft(p, rows_psi(c), c->twx, inv, 1.0f, B, c->st)) != cudaSuccess) return cuda_fail(c, e, "x");
-  if ((e = c->ky->lfft(p, lines_y(c, c->d.nx, c->d.nx, c->ncell), c->twy, inv, B, c->st)) != cudaSuccess)
+  if ((e = c->fx->fft(p, rows_psi(c), c->ftx, inv, 1.0f, B, c->st)) != cudaSuccess) return cuda_fail(c, e, "x");
+  if ((e = y_lines(c, p, lines_y(c, c->d.nx, c->d.nx, c->ncell), inv)) != cudaSuccess)
     return cuda_fail(c, e, "y");
-  if ((e = c->kz->lfft(p, lines_z(c, c->d.nx, c->d.nx, c->ncell), c->twz, inv, B, c->st)) != cudaSuccess)
+  if ((e = c->fz->line(p, lines_z(c, c->d.nx, c->d.nx, c->ncell), c->ftz, inv, B, c->st)) != cudaSuccess)
     return cuda_fail(c, e, "z");
   WDM_CU(c, cudaStreamSynchronize(c->st));
   return WDM_OK;
@@ -1639,6 +1727,28 @@ static wdm_status forward_boundary_to(wdm_ctx* c, int b, double dt, const float2
   return s;
 }
 
+// The Stockham passes' twiddles and schedule, made at the first adjoint (lam
+// and Hmu, not in use yet, stand in for psi and H in the timings).
+static wdm_status ensure_stockham(wdm_ctx* c) {
+  if (c->twz) return WDM_OK;
+  if (!c->twx) WDM_TRY(upload_twiddles(c, &c->twx, c->kx));
+  if (!c->twy) WDM_TRY(upload_twiddles(c, &c->twy, c->ky));
+  float4* tz = nullptr;
+  wdm_status s = upload_twiddles(c, &tz, c->kz);
+  c->twz = tz;
+  float2 *keep_psi = c->psi, *keep_H = c->H;
+  c->psi = c->lam;
+  c->H = c->Hmu;
+  if (s == WDM_OK) s = tune_passes(c);
+  c->psi = keep_psi;
+  c->H = keep_H;
+  if (s != WDM_OK && c->twz) {
+    cudaFree(c->twz);
+    c->twz = nullptr;
+  }
+  return s;
+}
+
 static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const float* rho_target, int where_t,
                                const double* tidal_dir, void* grad, int where_g, double* loss, double* damp) {
   WDM_TRY(need_psi(c));
@@ -1655,6 +1765,13 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
   if (!c->rho_t) WDM_TRY(dalloc(c, &c->rho_t, nc));
   if (!c->D6) WDM_TRY(dalloc(c, &c->D6, 6));
   if (!c->adj_acc) WDM_TRY(dalloc(c, &c->adj_acc, (size_t)2 * B));
+  // from here on the context runs the Stockham passes
+  struct Family {
+    wdm_ctx* c;
+    ~Family() { c->stockham = 0; }
+  } family{c};
+  c->stockham = 1;
+  WDM_TRY(ensure_stockham(c));
   const int nck = nsteps / ck + 1;
   const int last_seg = (nsteps - 1) / ck, jl0 = last_seg * ck;
   // Segment s keeps its states in slot set s % 2.  The recompute of segment
@@ -1906,7 +2023,7 @@ static bool persistent_ok(const wdm_group* g) {
 }
 
 // Member table of the persistent kernel for these time steps and mode: the
-// arguments of the direct x passes and the register-tile line passes that the
+// arguments of the row passes and the register-tile line passes that the
 // pass launches of step_impl would get.
 static wdm_status build_members(wdm_group* g, const std::vector<double>& dt, int mode,
                                 const std::vector<long long>& ver) {
@@ -1925,11 +2042,10 @@ static wdm_status build_members(wdm_group* g, const std::vector<double>& dt, int
     e.H = c->H;
     e.hpitch = c->hpitch;
     e.nhalf = c->nhalf;
-    e.twx = c->twx;
-    e.twy = c->twy;
-    e.twz = c->twz;
+    e.twx = c->ftx;
+    e.twy = c->fty;
+    e.twz = c->ftz;
     e.rows = rows_psi(c);
-    e.rows.impl = X_IMPL_DIRECT;
     e.ly_psi = lines_y(c, c->d.nx, c->d.nx, c->ncell);
     e.lz_psi = lines_z(c, c->d.nx, c->d.nx, c->ncell);
     e.ly_h = lines_y(c, c->nxh, c->hpitch, c->nhalf);
