@@ -121,7 +121,8 @@ __device__ __noinline__ void lines(float2* data, const LineGeom& g, const float4
   constexpr int SUB = ENS_THREADS / NT;
   static_assert(SUB * NT == ENS_THREADS, "tile groups fill the CTA");
   float4* tw = reinterpret_cast<float4*>(sm);
-  load_twiddles(tw, twg, N);  // visible after the first round's barrier
+  load_twiddles(tw, twg, N);
+  if (MODE == 1) __syncthreads();  // else visible after the first round's barrier
   const int sub = threadIdx.x / NT, tid = threadIdx.x % NT;
   float2* buf = reinterpret_cast<float2*>(sm) + 2 * N + (size_t)sub * N * LINES;
   const int tiles = (g.nlines + LINES - 1) / LINES;

@@ -2,6 +2,7 @@
 // factor_*.cu).
 #pragma once
 #include "factor_lines.cuh"
+#include "factor_planes.cuh"
 #include "factor_rows.cuh"
 #include "factor_set.h"
 #include "launch_util.cuh"
@@ -115,6 +116,44 @@ struct Launch {
                          const float4* tw, const float* shift, int batch, cudaStream_t st) {
     return rows<k_rows_r2c<N>>(rg, batch, st, in, H, rg, hpitch, hbstride, tw, shift);
   }
+  // Plane passes: one CTA per plane, with enough warps for 16 per SM (all that
+  // 128 registers a thread allow) over the CTAs that fit; all 16 in one CTA when
+  // there are no more planes than SMs.
+  static bool plane_ok(int ny) {
+    if constexpr (Plane<N>::KP == 0) return false;
+    else return plane_ny(ny) && plane_smem<N>(ny) <= PLANE_BYTES;
+  }
+  template <auto K, class Args>
+  static cudaError_t plane(const PlaneArgs& p, const Args& a, int batch, cudaStream_t st) {
+    cudaError_t e;
+    if ((e = prep_once<K>(PLANE_BYTES)) != cudaSuccess) return e;
+    const size_t smem = plane_smem<N>(p.rg.ny);
+    const int planes = p.rg.nrows / p.rg.ny * batch;
+    const int fit = (int)(228 * 1024 / (smem + 1024));
+    const int warps = planes <= sm_count() || fit <= 1 ? PLANE_WARPS : fit < 8 ? (PLANE_WARPS + fit - 1) / fit : 2;
+    K<<<planes, 32 * warps, smem, st>>>(p, a);
+    ++tl_kernel_launches;
+    return cudaGetLastError();
+  }
+  static cudaError_t plane_kick(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg,
+                                long long hpitch, long long hbstride, const float4* twx, const float4* twy,
+                                const KickArgs& a, bool fwd, int batch, cudaStream_t st) {
+    if constexpr (Plane<N>::KP == 0) {
+      return cudaErrorInvalidValue;
+    } else {
+      const PlaneArgs p{psi_in, psi, const_cast<float2*>(H), rg, hpitch, hbstride, twx, twy};
+      return fwd ? plane<k_plane_kick<N, true>>(p, a, batch, st) : plane<k_plane_kick<N, false>>(p, a, batch, st);
+    }
+  }
+  static cudaError_t plane_rho(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
+                               const float4* twx, const float4* twy, const RhoArgs& a, int batch, cudaStream_t st) {
+    if constexpr (Plane<N>::KP == 0) {
+      return cudaErrorInvalidValue;
+    } else {
+      const PlaneArgs p{psi, psi, H, rg, hpitch, hbstride, twx, twy};
+      return a.centre ? plane<k_plane_rho<N, true>>(p, a, batch, st) : plane<k_plane_rho<N, false>>(p, a, batch, st);
+    }
+  }
   static void fill_twiddles(float4* out) {
     fill_factor_twiddles<N>(out, [](long long m) {
       const double a = -2.0 * 3.14159265358979323846 * (double)m / (double)N;
@@ -122,7 +161,8 @@ struct Launch {
     });
   }
   static const FactorSet* set() {
-    static const FactorSet fs = {N, &line, &line_drift, &line_poisson, &fft, &rho, &kick, &c2r, &r2c, &fill_twiddles};
+    static const FactorSet fs = {N,    &line, &line_drift, &line_poisson, &fft,       &rho,          &kick,
+                                 &c2r, &r2c,  &plane_ok,   &plane_kick,   &plane_rho, &fill_twiddles};
     return &fs;
   }
 };

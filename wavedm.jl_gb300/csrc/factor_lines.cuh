@@ -104,14 +104,39 @@ __device__ __forceinline__ void op_points(const Op& op, float2* v, const typenam
 
 // MODE: 0 forward, 1 inverse, 2 forward / op / inverse (fused k-space step).
 //
-// The stages after stage A of a line in s (point p at s[p * LINES]; a
-// half-warp touches 16 neighbouring lines at one point, 128 contiguous bytes:
-// free of bank conflicts), the results to base[p * ps] (when ok).  freed:
-// called once the thread no longer needs s.
+// A forward transform runs stage A, then stage B; an inverse runs stage B's
+// transform on the frequencies k1 + RA k2 of each k1, then stage A's on the
+// elements (k1, n2) of each n2.  The first stage takes its points from load(p)
+// and leaves its elements in s (point p at s[p * LINES]; a half-warp touches 16
+// neighbouring lines at one point, 128 contiguous bytes: free of bank
+// conflicts).  In MODE 1 element (k1, n2) stays where frequency k1 + RA n2 was, so
+// that both stages work in place.
+template <int N, int MODE, class Load>
+__device__ __forceinline__ void line_begin(Load load, float2* s, const float4* tw, int t) {
+  using P = Plan<N>;
+  if constexpr (MODE == 1) {
+#pragma unroll 1
+    for (int i = 0; i < P::RA / P::T; ++i) {
+      const int k1 = t + P::T * i;
+      float2 v[P::RB];
+#pragma unroll
+      for (int k2 = 0; k2 < P::RB; ++k2) v[k2] = load(k1 + P::RA * k2);
+      dftR<P::RB, true>(v);
+      factor_twiddle<N, true>(v, tw, k1);
+#pragma unroll
+      for (int n2 = 0; n2 < P::RB; ++n2) s[(k1 + P::RA * n2) * LINES] = v[n2];
+    }
+  } else {
+    factor_a<N, false>(load, [&](int p, float2 v) { s[p * LINES] = v; }, t);
+  }
+}
+
+// The rest of the transform after a barrier: from s to base[p * ps] (when ok).
+// freed: called once the thread no longer needs s.
 template <int N, int MODE, bool TAB, class Op, class Hook>
 __device__ __forceinline__ void line_finish(float2* s, float2* base, long long ps, bool ok, const float4* tw,
-                                            const Op& op, const typename Op::Line& ln, const typename Op::Entry* tab, int t,
-                                            const Hook& freed) {
+                                            const Op& op, const typename Op::Line& ln, const typename Op::Entry* tab,
+                                            int t, const Hook& freed) {
   using P = Plan<N>;
   auto load = [&](int p) { return s[p * LINES]; };
   auto put = [&](int p, float2 v) {
@@ -130,8 +155,19 @@ __device__ __forceinline__ void line_finish(float2* s, float2* base, long long p
         t);
     __syncthreads();
     factor_a<N, true>(load, put, t);
+  } else if constexpr (MODE == 1) {
+#pragma unroll 1
+    for (int i = 0; i < P::RB / P::T; ++i) {
+      const int n2 = t + P::T * i;
+      float2 v[P::RA];
+#pragma unroll
+      for (int k1 = 0; k1 < P::RA; ++k1) v[k1] = load(k1 + P::RA * n2);
+      dftR<P::RA, true>(v);
+#pragma unroll
+      for (int n1 = 0; n1 < P::RA; ++n1) put(P::RB * n1 + n2, v[n1]);
+    }
   } else {
-    factor_b<N, MODE == 1>(
+    factor_b<N, false>(
         load, tw,
         [&](int k1, float2* v) {
 #pragma unroll
@@ -156,8 +192,7 @@ __device__ __forceinline__ void line_tile(float2* __restrict__ data, const LineG
   float2* base = data + b * g.bstride + (ok ? line_base(g, line) : 0);
   const int lc = ok ? line : 0;
   const typename Op::Line ln = op.line(g.x0 + lc % g.nxa, lc / g.nxa);
-  factor_a<N, MODE == 1>([&](int p) { return ok ? base[(long long)p * g.pstride] : make_float2(0.f, 0.f); },
-                         [&](int p, float2 v) { s[p * LINES + l] = v; }, t);
+  line_begin<N, MODE>([&](int p) { return ok ? base[(long long)p * g.pstride] : make_float2(0.f, 0.f); }, s + l, tw, t);
   __syncthreads();
   line_finish<N, MODE, false>(s + l, base, g.pstride, ok, tw, op, ln, nullptr, t, NoHook{});
 }
@@ -170,7 +205,8 @@ __global__ void __launch_bounds__(line_threads<N>(), line_ctas<N>())
 k_line_tile(float2* __restrict__ data, LineGeom g, const float4* __restrict__ twg, Op op) {
   extern __shared__ float2 smem[];
   float4* tw = reinterpret_cast<float4*>(smem);
-  load_twiddles(tw, twg, N);  // visible after the tile's first barrier
+  load_twiddles(tw, twg, N);
+  if (MODE == 1) __syncthreads();  // else visible after the tile's first barrier
   line_tile<N, MODE, Op>(data, g, tw, op, blockIdx.x * LINES, blockIdx.y, smem + 2 * N, threadIdx.x);
 }
 
@@ -326,7 +362,7 @@ k_line_tma(float2* __restrict__ data, const __grid_constant__ CUtensorMap map, c
       }
     };
     float2* sl = s + l;
-    factor_a<N, MODE == 1>([&](int p) { return sl[p * LINES]; }, [&](int p, float2 v) { sl[p * LINES] = v; }, t);
+    line_begin<N, MODE>([&](int p) { return sl[p * LINES]; }, sl, tw, t);
     __syncthreads();
     line_finish<N, MODE, STAGED>(sl, base, g.pstride, ok, tw, op, ln, optab, t, refill);
     if constexpr (SLOTS == 2 && !LATE) {

@@ -125,63 +125,85 @@ __device__ __forceinline__ void b_items(const Warp<N>& w, Item item) {
   }
 }
 
-// Stage B's transform of a row's frequencies k1 + RA k2 (in v) into the elements
-// (k1, n2) of the buffer row: the first half of an inverse.
+// Stage B's transform of a row's frequencies k1 + RA k2 (in v) into its elements
+// (k1, n2) at d: the first half of an inverse.
 template <int N>
-__device__ __forceinline__ void b_inverse(const Warp<N>& w, float2* v, int j, int k1) {
+__device__ __forceinline__ void b_inverse(const float4* tw, float2* v, float2* d, int k1) {
   constexpr int RB = Rows<N>::RB;
   dftR<RB, true>(v);
-  factor_twiddle<N, true>(v, w.tw, k1);
-  float2* d = w.row(j, k1);
+  factor_twiddle<N, true>(v, tw, k1);
 #pragma unroll
   for (int n2 = 0; n2 < RB; ++n2) d[n2] = v[n2];
 }
 
-// Stage B of a transform: the elements (k1, n2) of a buffer row into its
-// frequencies k1 + RA k2 (in v).
+// Stage B of a transform: a row's elements (k1, n2) at s into its frequencies
+// k1 + RA k2 (in v).
 template <int N, bool INV>
-__device__ __forceinline__ void b_forward(const Warp<N>& w, float2* v, int j, int k1) {
+__device__ __forceinline__ void b_forward(const float4* tw, float2* v, const float2* s, int k1) {
   constexpr int RB = Rows<N>::RB;
-  const float2* s = w.row(j, k1);
 #pragma unroll
   for (int n2 = 0; n2 < RB; ++n2) v[n2] = s[n2];
-  factor_twiddle<N, INV>(v, w.tw, k1);
+  factor_twiddle<N, INV>(v, tw, k1);
   dftR<RB, INV>(v);
 }
 
-// The pairs' packed lines A + iB from their half spectra, through stage B into
-// E(0): Z[p] = A[p] + iB[p], Z[N - p] = conj A[p] + i conj B[p].
+// The frequencies k1 + RA k2 of a packed line A + iB from the half spectra of its
+// rows: Z[p] = A[p] + iB[p], Z[N - p] = conj A[p] + i conj B[p].
+template <int N>
+__device__ __forceinline__ void pack_half(float2* v, const float2* ha, const float2* hb, bool ok, int k1) {
+  constexpr int RA = Rows<N>::RA, RB = Rows<N>::RB;
+#pragma unroll
+  for (int k2 = 0; k2 < RB; ++k2) {
+    // the frequency lies below N/2 for k2 < RB/2, above for k2 > RB/2
+    const int k = k1 + RA * k2;
+    const bool low = k2 < RB / 2 || (k2 == RB / 2 && k1 == 0);
+    const int q = low ? k : N - k;
+    float2 a = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
+    if (ok) {
+      a = ha[q];
+      c = hb[q];
+    }
+    v[k2] = low ? fma2(swapped(c), make_float2(-1.f, 1.f), a) : fma2(a, make_float2(1.f, -1.f), swapped(c));
+  }
+}
+
+// The half spectra of a pair's rows at the frequencies of the packed line's
+// butterflies k1 (va) and its partner (vb: RA - k1, or RA/2 for k1 = 0, which is
+// its own partner as RA/2 is): between them they hold the frequencies k and N -
+// k.  put(k, a, b): rows A and B at frequency k.
+template <int N, class Put>
+__device__ __forceinline__ void split_half(const float2* va, const float2* vb, int k1, Put put) {
+  constexpr int RA = Rows<N>::RA, RB = Rows<N>::RB;
+  const bool self = k1 == 0;
+  const int kb = self ? RA / 2 : RA - k1;
+  auto out = [&](int k, float2 z, float2 zn) {  // zn: the packed line at N - k
+    put(k, cscale(fma2(zn, make_float2(1.f, -1.f), z), 0.5f),
+        cscale(fma2(swapped(z), make_float2(1.f, -1.f), swapped(zn)), 0.5f));
+  };
+#pragma unroll
+  for (int k2 = 0; k2 < RB / 2; ++k2) {
+    out(k1 + RA * k2, va[k2], self ? va[(RB - k2) % RB] : vb[RB - 1 - k2]);
+    out(kb + RA * k2, vb[k2], self ? vb[RB - 1 - k2] : va[RB - 1 - k2]);
+  }
+  if (self) out(N / 2, va[RB / 2], va[RB / 2]);
+}
+
+// The pairs' packed lines from their half spectra, through stage B into E(0).
 template <int N>
 __device__ __forceinline__ void packed_in(const Warp<N>& w, const float2* __restrict__ H, long long hpitch,
                                           long long hbstride) {
   using R = Rows<N>;
-  constexpr int RA = R::RA, RB = R::RB;
   b_items<N, R::PW>(w, [&](int j, int k1) {
     int b, ra;
     const bool ok = w.pair(j, &b, &ra);
     const float2* ha = H + b * hbstride + ra * hpitch;
-    const float2* hb = ha + hpitch;
-    float2 v[RB];
-#pragma unroll
-    for (int k2 = 0; k2 < RB; ++k2) {
-      // the frequency lies below N/2 for k2 < RB/2, above for k2 > RB/2
-      const int k = k1 + RA * k2;
-      const bool low = k2 < RB / 2 || (k2 == RB / 2 && k1 == 0);
-      const int q = low ? k : N - k;
-      float2 a = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
-      if (ok) {
-        a = ha[q];
-        c = hb[q];
-      }
-      v[k2] = low ? fma2(swapped(c), make_float2(-1.f, 1.f), a) : fma2(a, make_float2(1.f, -1.f), swapped(c));
-    }
-    b_inverse(w, v, j, k1);
+    float2 v[R::RB];
+    pack_half<N>(v, ha, ha + hpitch, ok, k1);
+    b_inverse<N>(w.tw, v, w.row(j, k1), k1);
   });
 }
 
-// The half spectra of the pairs' rows from their packed lines in E(0): stage B
-// of the butterflies k1 and RA - k1 (0 and RA/2) in one lane, which between them
-// hold the frequencies k and N - k.
+// The half spectra of the pairs' rows from their packed lines in E(0).
 template <int N>
 __device__ __forceinline__ void packed_out(const Warp<N>& w, float2* __restrict__ H, long long hpitch,
                                            long long hbstride) {
@@ -191,26 +213,17 @@ __device__ __forceinline__ void packed_out(const Warp<N>& w, float2* __restrict_
   for (int i = 0; i < (ITEMS + 31) / 32; ++i) {
     const int q = w.lane + 32 * i;
     if (ITEMS % 32 != 0 && q >= ITEMS) break;
-    const int j = q / (RA / 2), k1 = q % (RA / 2);
-    const bool self = k1 == 0;  // 0 and RA/2 are each their own partner
-    const int kb = self ? RA / 2 : RA - k1;
+    const int j = q / (RA / 2), k1 = q % (RA / 2), kb = k1 ? RA - k1 : RA / 2;
     float2 va[RB], vb[RB];
-    b_forward<N, false>(w, va, j, k1);
-    b_forward<N, false>(w, vb, j, kb);
+    b_forward<N, false>(w.tw, va, w.row(j, k1), k1);
+    b_forward<N, false>(w.tw, vb, w.row(j, kb), kb);
     int b, ra;
     if (!w.pair(j, &b, &ra)) continue;
     float2* ha = H + b * hbstride + ra * hpitch;
-    float2* hb = ha + hpitch;
-    auto put = [&](int k, float2 z, float2 zn) {  // zn: the packed line at N - k
-      ha[k] = cscale(fma2(zn, make_float2(1.f, -1.f), z), 0.5f);
-      hb[k] = cscale(fma2(swapped(z), make_float2(1.f, -1.f), swapped(zn)), 0.5f);
-    };
-#pragma unroll
-    for (int k2 = 0; k2 < RB / 2; ++k2) {
-      put(k1 + RA * k2, va[k2], self ? va[(RB - k2) % RB] : vb[RB - 1 - k2]);
-      put(kb + RA * k2, vb[k2], self ? vb[RB - 1 - k2] : va[RB - 1 - k2]);
-    }
-    if (self) put(N / 2, va[RB / 2], va[RB / 2]);
+    split_half<N>(va, vb, k1, [&](int k, float2 x, float2 y) {
+      ha[k] = x;
+      ha[hpitch + k] = y;
+    });
   }
 }
 
@@ -285,6 +298,48 @@ __device__ __forceinline__ void kick_row_points(float2* x, float* phi, const flo
   }
 }
 
+// The points RB n1 + n2 of a row (row: its point n2).
+template <int N>
+__device__ __forceinline__ void load_points(float2* x, const float2* row, bool ok) {
+#pragma unroll
+  for (int n1 = 0; n1 < Rows<N>::RA; ++n1) x[n1] = ok ? row[Rows<N>::RB * n1] : make_float2(0.f, 0.f);
+}
+
+// The kick of one pair by an A lane: the packed potential line's elements (k1,
+// n2) at (0, k1), x: row A's points of psi.  FWD: the kicked rows' elements to
+// at(half, k1); else the kicked rows to psi.  base: the offset of row A's point
+// n2 in psi_in and psi.
+template <int N, bool FWD, class At>
+__device__ __forceinline__ void kick_lane(At at, float2* x, const float2* psi_in, float2* psi, long long base,
+                                          const RowGeom& rg, int b, int ra, bool ok, int n2, const float* T6,
+                                          const KickArgs& a) {
+  using R = Rows<N>;
+  constexpr int RA = R::RA, RB = R::RB;
+  float2 z[RA];  // (Phi of row A, Phi of row B)
+#pragma unroll
+  for (int k1 = 0; k1 < RA; ++k1) z[k1] = *at(0, k1);
+  dftR<RA, true>(z);
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    const int r = ra + half;
+    float phi[RA];
+#pragma unroll
+    for (int n1 = 0; n1 < RA; ++n1) phi[n1] = half ? z[n1].y : z[n1].x;
+    const float* vrow = a.V && ok ? a.V + b * a.v_bstride + (long long)r * rg.pitch : nullptr;
+    kick_row_points<RA>(x, phi, T6, a, r % rg.ny, r / rg.ny, vrow, [&](int n1) { return RB * n1 + n2; });
+    if constexpr (FWD) {
+      dftR<RA, false>(x);
+#pragma unroll
+      for (int k1 = 0; k1 < RA; ++k1) *at(half, k1) = x[k1];
+    } else {
+      if (ok)
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) psi[base + half * rg.pitch + RB * n1] = x[n1];
+    }
+    if (half == 0) load_points<N>(x, psi_in + base + rg.pitch, ok);
+  }
+}
+
 template <int N, bool FWD>
 __device__ __forceinline__ void kick_units(Warp<N>& w, const float2* psi_in, float2* psi, const float2* __restrict__ H,
                                            const RowGeom& rg, long long hpitch, long long hbstride, const KickArgs& a) {
@@ -295,43 +350,17 @@ __device__ __forceinline__ void kick_units(Warp<N>& w, const float2* psi_in, flo
     int b, ra;
     const bool ok = w.pair(w.pr, &b, &ra);
     const long long base = b * rg.bstride + (long long)ra * rg.pitch + w.n2;
-    auto pos = [&](int n1) { return RB * n1 + w.n2; };
     float2 x[RA];
-#pragma unroll
-    for (int n1 = 0; n1 < RA; ++n1) x[n1] = ok ? psi_in[base + RB * n1] : make_float2(0.f, 0.f);
+    load_points<N>(x, psi_in + base, ok);
     float T6[10];
     kick_tidal<N>(T6, a, rg, b);
     __syncwarp();
-    float2 z[RA];  // (Phi of row A, Phi of row B)
-#pragma unroll
-    for (int k1 = 0; k1 < RA; ++k1) z[k1] = *w.at(0, k1);
-    dftR<RA, true>(z);
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      const int r = ra + half;
-      float phi[RA];
-#pragma unroll
-      for (int n1 = 0; n1 < RA; ++n1) phi[n1] = half ? z[n1].y : z[n1].x;
-      const float* vrow = a.V && ok ? a.V + b * a.v_bstride + (long long)r * rg.pitch : nullptr;
-      kick_row_points<RA>(x, phi, T6, a, r % rg.ny, r / rg.ny, vrow, pos);
-      if constexpr (FWD) {
-        dftR<RA, false>(x);
-#pragma unroll
-        for (int k1 = 0; k1 < RA; ++k1) *w.at(half, k1) = x[k1];
-      } else {
-        if (ok)
-#pragma unroll
-          for (int n1 = 0; n1 < RA; ++n1) psi[base + half * rg.pitch + RB * n1] = x[n1];
-      }
-      if (half == 0)
-#pragma unroll
-        for (int n1 = 0; n1 < RA; ++n1) x[n1] = ok ? psi_in[base + rg.pitch + RB * n1] : make_float2(0.f, 0.f);
-    }
+    kick_lane<N, FWD>([&](int half, int k1) { return w.at(half, k1); }, x, psi_in, psi, base, rg, b, ra, ok, w.n2, T6, a);
     __syncwarp();
     if constexpr (FWD) {
       b_items<N, 2 * R::PW>(w, [&](int j, int k1) {
         float2 v[RB];
-        b_forward<N, false>(w, v, j, k1);
+        b_forward<N, false>(w.tw, v, w.row(j, k1), k1);
         int ib, ir;
         if (!w.pair(j % R::PW, &ib, &ir)) return;
         float2* row = psi + ib * rg.bstride + (long long)(ir + j / R::PW) * rg.pitch + k1;
@@ -392,6 +421,70 @@ __device__ __forceinline__ void rows_centre_done(const RhoArgs& a, const RowGeom
   }
 }
 
+// The density of one pair by an A lane: psi from the elements at(half, k1)
+// (write_psi: inverted, masked and stored at base) or from base; the packed
+// (rho_A, rho_B) line's elements to at(0, k1).  base: row A's point n2 in psi.
+template <int N, bool CEN, class At>
+__device__ __forceinline__ void rho_lane(At at, float2* base, const RowGeom& rg, int b, int ra, bool ok, int n2,
+                                         float shift, const RhoArgs& a, CentreAcc& ca) {
+  using R = Rows<N>;
+  constexpr int RA = R::RA, RB = R::RB;
+  float d0[RA];   // the density of row A
+  float2 z[RA];   // (rho_A, rho_B)
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    const int r = ra + half;
+    float2* row = base + half * rg.pitch;
+    float2 v[RA];
+    if (a.write_psi) {
+#pragma unroll
+      for (int k1 = 0; k1 < RA; ++k1) v[k1] = *at(half, k1);
+      dftR<RA, true>(v);
+      if (a.mx) {
+        const float myz = ok ? a.my[r % rg.ny] * a.mz[r / rg.ny] : 0.f;
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) v[n1] = cscale(v[n1], myz * a.mx[RB * n1 + n2]);
+      }
+      if (ok)
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) row[RB * n1] = v[n1];
+    } else {
+      load_points<N>(v, row, ok);
+    }
+    // each optional step is tested once for the row's points
+    float d[RA];
+#pragma unroll
+    for (int n1 = 0; n1 < RA; ++n1) d[n1] = fmaf(v[n1].x, v[n1].x, v[n1].y * v[n1].y);
+    if (ok && a.nonfinite) {
+      bool bad = false;
+#pragma unroll
+      for (int n1 = 0; n1 < RA; ++n1) bad |= !isfinite(d[n1]);
+      if (bad) *a.nonfinite = 1;
+    }
+    if constexpr (CEN) {
+#pragma unroll
+      for (int n1 = 0; n1 < RA; ++n1) {
+        const int x = RB * n1 + n2;
+        ca.add(d[n1], (unsigned)r * (unsigned)N + (unsigned)x, x, half);
+      }
+    }
+    // rows without baryon mass are zero and not read
+    if (ok && a.rho_b && (!a.rb_rows || a.rb_rows[r])) {
+      const float* rb = a.rho_b + b * a.rb_bstride + (long long)r * rg.pitch + n2;
+#pragma unroll
+      for (int n1 = 0; n1 < RA; ++n1) d[n1] += rb[RB * n1];
+    }
+#pragma unroll
+    for (int n1 = 0; n1 < RA; ++n1) {
+      if (half == 0) d0[n1] = d[n1] - shift;
+      else z[n1] = make_float2(d0[n1], d[n1] - shift);
+    }
+  }
+  dftR<RA, false>(z);
+#pragma unroll
+  for (int k1 = 0; k1 < RA; ++k1) *at(0, k1) = z[k1];
+}
+
 template <int N, bool CEN>
 __device__ __forceinline__ void rho_units(Warp<N>& w, float2* __restrict__ psi, float2* __restrict__ H,
                                           const RowGeom& rg, long long hpitch, long long hbstride, const RhoArgs& a) {
@@ -408,72 +501,18 @@ __device__ __forceinline__ void rho_units(Warp<N>& w, float2* __restrict__ psi, 
         float2 v[RB];
 #pragma unroll
         for (int k2 = 0; k2 < RB; ++k2) v[k2] = iok ? row[RA * k2] : make_float2(0.f, 0.f);
-        b_inverse(w, v, j, k1);
+        b_inverse<N>(w.tw, v, w.row(j, k1), k1);
       });
       __syncwarp();
     }
     int b, ra;
     const bool ok = w.pair(w.pr, &b, &ra);
     const float shift = a.shift ? a.shift[b] : 0.f;
-    float2* base = psi + b * rg.bstride + (long long)ra * rg.pitch + w.n2;
     CentreAcc ca;
     ca.reset();
-    float d0[RA];   // the density of row A
-    float2 z[RA];   // (rho_A, rho_B)
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      const int r = ra + half;
-      float2* row = base + half * rg.pitch;
-      float2 v[RA];
-      if (a.write_psi) {
-#pragma unroll
-        for (int k1 = 0; k1 < RA; ++k1) v[k1] = *w.at(half, k1);
-        dftR<RA, true>(v);
-        if (a.mx) {
-          const float myz = ok ? a.my[r % rg.ny] * a.mz[r / rg.ny] : 0.f;
-#pragma unroll
-          for (int n1 = 0; n1 < RA; ++n1) v[n1] = cscale(v[n1], myz * a.mx[RB * n1 + w.n2]);
-        }
-        if (ok)
-#pragma unroll
-          for (int n1 = 0; n1 < RA; ++n1) row[RB * n1] = v[n1];
-      } else {
-#pragma unroll
-        for (int n1 = 0; n1 < RA; ++n1) v[n1] = ok ? row[RB * n1] : make_float2(0.f, 0.f);
-      }
-      // each optional step is tested once for the row's points
-      float d[RA];
-#pragma unroll
-      for (int n1 = 0; n1 < RA; ++n1) d[n1] = fmaf(v[n1].x, v[n1].x, v[n1].y * v[n1].y);
-      if (ok && a.nonfinite) {
-        bool bad = false;
-#pragma unroll
-        for (int n1 = 0; n1 < RA; ++n1) bad |= !isfinite(d[n1]);
-        if (bad) *a.nonfinite = 1;
-      }
-      if constexpr (CEN) {
-#pragma unroll
-        for (int n1 = 0; n1 < RA; ++n1) {
-          const int x = RB * n1 + w.n2;
-          ca.add(d[n1], (unsigned)r * (unsigned)N + (unsigned)x, x, half);
-        }
-      }
-      // rows without baryon mass are zero and not read
-      if (ok && a.rho_b && (!a.rb_rows || a.rb_rows[r])) {
-        const float* rb = a.rho_b + b * a.rb_bstride + (long long)r * rg.pitch + w.n2;
-#pragma unroll
-        for (int n1 = 0; n1 < RA; ++n1) d[n1] += rb[RB * n1];
-      }
-#pragma unroll
-      for (int n1 = 0; n1 < RA; ++n1) {
-        if (half == 0) d0[n1] = d[n1] - shift;
-        else z[n1] = make_float2(d0[n1], d[n1] - shift);
-      }
-    }
+    rho_lane<N, CEN>([&](int half, int k1) { return w.at(half, k1); },
+                     psi + b * rg.bstride + (long long)ra * rg.pitch + w.n2, rg, b, ra, ok, w.n2, shift, a, ca);
     if constexpr (CEN) rows_centre_done<N>(a, rg, ca, cs, b, ra, ok, w.n2);
-    dftR<RA, false>(z);
-#pragma unroll
-    for (int k1 = 0; k1 < RA; ++k1) *w.at(0, k1) = z[k1];
     __syncwarp();
     packed_out<N>(w, H, hpitch, hbstride);
     __syncwarp();
@@ -518,7 +557,7 @@ k_rows_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg
     __syncwarp();
     b_items<N, 2 * R::PW>(w, [&](int j, int k1) {
       float2 v[RB];
-      b_forward<N, INV>(w, v, j, k1);
+      b_forward<N, INV>(w.tw, v, w.row(j, k1), k1);
       int ib, ir;
       if (!w.pair(j % R::PW, &ib, &ir)) return;
       float2* row = data + ib * rg.bstride + (long long)(ir + j / R::PW) * rg.pitch + k1;

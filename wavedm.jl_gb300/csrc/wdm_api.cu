@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -128,6 +129,8 @@ struct Profiler {
   struct Rec {
     int pass;
     cudaEvent_t a, b;
+    double share;  // of the interval (a launch that holds several passes)
+    bool last;     // the events go back to the pool with this record
   };
   std::vector<Rec> pending;
   int64_t launches[NPASS] = {0};
@@ -156,6 +159,9 @@ struct wdm_ctx {
   float4 *ftx = nullptr, *fty = nullptr, *ftz = nullptr;
   const KernelSet *kx = nullptr, *ky = nullptr, *kz = nullptr;
   int stockham = 0;  // set while the adjoint runs
+  int planes = 0;    // the step runs on plane passes (y transforms inside the kick and the density pass)
+  int h_y = 0;       // H holds the potential y-spectral (left so by a plane density pass)
+  int psi_y = 0;     // psi is y-spectral as well as x-spectral, between a kick and a density pass
   double dx = 0, dy = 0, dz = 0, x0 = 0, y0 = 0, z0 = 0;
   // device buffers
   float2* psi = nullptr;
@@ -243,8 +249,9 @@ static cudaError_t prof_flush(wdm_ctx* c) {
   if (e != cudaSuccess) return e;
   for (auto& r : c->prof.pending) {
     float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, r.a, r.b) == cudaSuccess) c->prof.ms[r.pass] += ms;
+    if (cudaEventElapsedTime(&ms, r.a, r.b) == cudaSuccess) c->prof.ms[r.pass] += ms * r.share;
     c->prof.launches[r.pass] += 1;
+    if (!r.last) continue;
     c->prof.pool.push_back(r.a);
     c->prof.pool.push_back(r.b);
   }
@@ -263,6 +270,33 @@ static cudaError_t counted(wdm_ctx* c, F launch) {
   return e;
 }
 
+static double pass_bytes(const wdm_ctx* c, int p);
+
+// A launch that holds the given passes: each counts one launch and its share,
+// by algorithmic bytes, of the launch's time.
+template <class F>
+static cudaError_t run_passes(wdm_ctx* c, std::initializer_list<int> passes, F launch) {
+  uint64_t in = 0;
+  double bytes = 0.0;
+  for (int p : passes) {
+    in |= 1ull << p;
+    bytes += pass_bytes(c, p);
+  }
+  if (!c->prof.on || !(c->prof.mask & in)) return counted(c, launch);
+  cudaEvent_t a = prof_event(c), b = prof_event(c);
+  cudaEventRecord(a, c->st);
+  cudaError_t e = counted(c, launch);
+  cudaEventRecord(b, c->st);
+  for (int p : passes)
+    if ((c->prof.mask >> p) & 1ull) c->prof.pending.push_back({p, a, b, pass_bytes(c, p) / bytes, false});
+  c->prof.pending.back().last = true;
+  if (c->prof.pending.size() > 4096) {
+    cudaError_t f = prof_flush(c);
+    if (e == cudaSuccess) e = f;
+  }
+  return e;
+}
+
 template <class F>
 static cudaError_t run_pass(wdm_ctx* c, int pass, F launch) {
   if (!c->prof.on || !((c->prof.mask >> pass) & 1ull)) return counted(c, launch);
@@ -270,7 +304,7 @@ static cudaError_t run_pass(wdm_ctx* c, int pass, F launch) {
   cudaEventRecord(a, c->st);
   cudaError_t e = counted(c, launch);
   cudaEventRecord(b, c->st);
-  c->prof.pending.push_back({pass, a, b});
+  c->prof.pending.push_back({pass, a, b, 1.0, true});
   if (c->prof.pending.size() > 4096) {
     cudaError_t f = prof_flush(c);
     if (e == cudaSuccess) e = f;
@@ -555,7 +589,6 @@ static cudaError_t x_kick(wdm_ctx* c, const float2* in, const KickArgs& a, bool 
                      : c->fx->kick(in, c->psi, c->H, rows_psi(c), c->hpitch, c->nhalf, c->ftx, a, fwd, c->d.batch, c->st);
 }
 
-// density (+baryons) of psi -> H, then the Poisson solve on H (P5..P8).
 // The CIC deposit of the current particles into rho_b (zero before it), made
 // once per particle set.
 static wdm_status ensure_deposit(wdm_ctx* c) {
@@ -568,7 +601,16 @@ static wdm_status ensure_deposit(wdm_ctx* c) {
   return WDM_OK;
 }
 
-// Density pass (P5) and Poisson solve (P6-P8).  write_psi != 0: psi holds
+// The potential's y inverse (P8): H from y-spectral to rows.
+static wdm_status potential_rows(wdm_ctx* c) {
+  cudaError_t e = run_pass(c, P_H_Y_INV, [&] { return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), true); });
+  if (e != cudaSuccess) return cuda_fail(c, e, "H y inv");
+  c->h_y = 0;
+  return WDM_OK;
+}
+
+// Density pass (P5) and Poisson solve (P6-P8).  On plane passes P4, P5 and P6 are
+// one launch, and P8 is left to the kick (h_y).  write_psi != 0: psi holds
 // x-spectral data (after P4); the pass inverts it first (with the absorbing
 // mask) and writes real-space psi back.  With baryons, P5 adds the kept
 // deposit (only the rows it flags are read).
@@ -592,13 +634,23 @@ static wdm_status density_poisson(wdm_ctx* c, int write_psi, double dt_mask) {
     WDM_CU(c, cudaMemsetAsync(c->centre, 0, sizeof(unsigned long long) * CENTRE_WORDS * B, c->st));
     ra.centre = c->centre;
   }
-  cudaError_t e = run_pass(c, write_psi ? P_X_INV_RHO : P_DENSITY, [&] {
-    return x_rho(c, ra, c->nparts > 0 ? LP_X_RHO_B : LP_X_RHO);
-  });
-  if (e != cudaSuccess) return cuda_fail(c, e, "x_inv_rho");
-  if ((e = run_pass(c, P_H_Y_FWD, [&] { return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), false); })) !=
-      cudaSuccess)
-    return cuda_fail(c, e, "H y fwd");
+  cudaError_t e;
+  const bool planes = c->planes && !c->stockham && (!write_psi || c->psi_y);
+  if (planes) {
+    auto launch = [&] {
+      return c->fx->plane_rho(c->psi, c->H, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->fty, ra, B, c->st);
+    };
+    e = write_psi ? run_passes(c, {P_PSI_Y_INV, P_X_INV_RHO, P_H_Y_FWD}, launch)
+                  : run_passes(c, {P_DENSITY, P_H_Y_FWD}, launch);
+    if (e != cudaSuccess) return cuda_fail(c, e, "plane density");
+    c->psi_y = 0;
+  } else {
+    e = run_pass(c, write_psi ? P_X_INV_RHO : P_DENSITY, [&] { return x_rho(c, ra, c->nparts > 0 ? LP_X_RHO_B : LP_X_RHO); });
+    if (e != cudaSuccess) return cuda_fail(c, e, "x_inv_rho");
+    if ((e = run_pass(c, P_H_Y_FWD, [&] { return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), false); })) !=
+        cudaSuccess)
+      return cuda_fail(c, e, "H y fwd");
+  }
   PoissonOp po;
   po.kx2 = c->kx2;
   po.ky2 = c->ky2;
@@ -608,9 +660,8 @@ static wdm_status density_poisson(wdm_ctx* c, int write_psi, double dt_mask) {
                     [&] { return z_poisson(c, c->H, lines_z(c, c->nxh, c->hpitch, c->nhalf), po); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "H z poisson");
-  if ((e = run_pass(c, P_H_Y_INV, [&] { return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), true); })) !=
-      cudaSuccess)
-    return cuda_fail(c, e, "H y inv");
+  c->h_y = planes;
+  if (!planes) WDM_TRY(potential_rows(c));
   c->phi_valid = 1;
   return WDM_OK;
 }
@@ -690,9 +741,17 @@ static wdm_status kick(wdm_ctx* c, double dt, int sched_row, bool fwd, const flo
     if (e != cudaSuccess) return cuda_fail(c, e, "tide frame");
   }
   const float2* in = psi_in ? psi_in : c->psi;
-  cudaError_t e = run_pass(c, fwd ? P_KICK_FWD : P_KICK, [&] {
-    return x_kick(c, in, a, fwd);
-  });
+  cudaError_t e;
+  if (c->h_y) {  // left by a plane density pass: the plane kick takes it from there
+    auto launch = [&] {
+      return c->fx->plane_kick(in, c->psi, c->H, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->fty, a, fwd, c->d.batch, c->st);
+    };
+    e = fwd ? run_passes(c, {P_H_Y_INV, P_KICK_FWD, P_PSI_Y_FWD}, launch) : run_pass(c, P_KICK, launch);
+    if (e != cudaSuccess) return cuda_fail(c, e, "plane kick");
+    c->psi_y = fwd;
+    return WDM_OK;
+  }
+  e = run_pass(c, fwd ? P_KICK_FWD : P_KICK, [&] { return x_kick(c, in, a, fwd); });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_kick");
   return WDM_OK;
 }
@@ -717,7 +776,8 @@ static wdm_status drift_yz(wdm_ctx* c, double dt, float sign = 1.f, float2* data
   op.scale = (float)(1.0 / ((double)c->d.nx * c->d.ny * c->d.nz));
   op.precise = precise;
   cudaError_t e;
-  if ((e = run_pass(c, P_PSI_Y_FWD,
+  const bool psi_y = c->psi_y && !data;  // a plane kick has done the y transform
+  if (!psi_y && (e = run_pass(c, P_PSI_Y_FWD,
                     [&] { return y_lines(c, psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), false); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "psi y fwd");
@@ -725,6 +785,11 @@ static wdm_status drift_yz(wdm_ctx* c, double dt, float sign = 1.f, float2* data
                     [&] { return z_drift(c, psi, lines_z(c, c->d.nx, c->d.nx, c->ncell), op); })) !=
       cudaSuccess)
     return cuda_fail(c, e, "psi z drift");
+  // the plane density pass takes psi y-spectral
+  if (c->planes && !c->stockham) {
+    c->psi_y = 1;
+    return WDM_OK;
+  }
   if ((e = run_pass(c, P_PSI_Y_INV,
                     [&] { return y_lines(c, psi, lines_y(c, c->d.nx, c->d.nx, c->ncell), true); })) !=
       cudaSuccess)
@@ -815,6 +880,7 @@ wdm_status wdm_destroy(wdm_ctx* c) {
   for (cudaEvent_t e : {c->ev_ck, c->ev_rec[0], c->ev_rec[1], c->ev_bwd[0], c->ev_bwd[1]})
     if (e) cudaEventDestroy(e);
   for (auto& r : c->prof.pending) {
+    if (!r.last) continue;
     cudaEventDestroy(r.a);
     cudaEventDestroy(r.b);
   }
@@ -1058,6 +1124,8 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
     return bail(WDM_ERR_CUDA);
   }
   if ((s = tune_passes(c)) != WDM_OK) return bail(s);
+  const char* planes_env = std::getenv("WDM_PLANES");  // "off": the separate passes (tests, profiling)
+  c->planes = c->fx->plane_ok(d->ny) && !(planes_env && !std::strcmp(planes_env, "off"));
   if ((e = cudaStreamSynchronize(c->st)) != cudaSuccess) {
     cuda_fail(c, e, "sync");
     return bail(WDM_ERR_CUDA);
@@ -1074,6 +1142,7 @@ wdm_status wdm_set_psi(wdm_ctx* c, const void* psi, int32_t where) {
   WDM_TRY(update_shift(c));
   c->have_psi = 1;
   c->phi_valid = 0;
+  c->psi_y = 0;
   return WDM_OK;
 }
 
@@ -1093,8 +1162,19 @@ wdm_status wdm_get_rho(wdm_ctx* c, float* rho, int32_t where) {
 static wdm_status phi_real(wdm_ctx* c) {
   WDM_TRY(ensure_scratch(c));
   if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, 0.0));
+  // a y-spectral H stays as it is (the next kick and captured graphs start from it)
+  float2* H = c->H;
+  if (c->h_y) {
+    WDM_CU(c, cudaMemcpyAsync(c->scratch_h, c->H, sizeof(float2) * c->nhalf * c->d.batch, cudaMemcpyDeviceToDevice, c->st));
+    c->H = c->scratch_h;
+    wdm_status s = potential_rows(c);
+    c->H = H;
+    c->h_y = 1;
+    WDM_TRY(s);
+    H = c->scratch_h;
+  }
   cudaError_t e = run_pass(c, P_PHI_OUT, [&] {
-    return c->fx->c2r(c->H, c->scratch_f, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
+    return c->fx->c2r(H, c->scratch_f, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
   });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_c2r");
   return WDM_OK;
@@ -1770,6 +1850,7 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
     wdm_ctx* c;
     ~Family() { c->stockham = 0; }
   } family{c};
+  if (c->phi_valid && c->h_y) WDM_TRY(potential_rows(c));
   c->stockham = 1;
   WDM_TRY(ensure_stockham(c));
   const int nck = nsteps / ck + 1;
@@ -2105,6 +2186,19 @@ static wdm_status build_members(wdm_group* g, const std::vector<double>& dt, int
   return WDM_OK;
 }
 
+// H as the schedule starts from it (a captured sequence holds the state it was
+// captured in): y-spectral where the member steps on plane passes, rows for the
+// persistent kernel.  On stream st.
+static wdm_status start_state(wdm_ctx* c, cudaStream_t st, int sched) {
+  const bool want = sched != GROUP_PERSISTENT && c->planes;
+  if ((c->h_y != 0) == want) return WDM_OK;
+  cudaStream_t own = c->st;
+  c->st = st;
+  wdm_status s = want ? density_poisson(c, 0, 0.0) : potential_rows(c);
+  c->st = own;
+  return s;
+}
+
 // Enqueue one call on the group's stream under schedule `sched`: the captured
 // graph of the members' pass launches, or the graph of one persistent launch
 // (its barrier words cleared first).  Graphs are captured once per (nsteps,
@@ -2112,6 +2206,10 @@ static wdm_status build_members(wdm_group* g, const std::vector<double>& dt, int
 static wdm_status group_launch(wdm_group* g, int32_t nsteps, const std::vector<double>& dt,
                                const std::vector<long long>& ver, int32_t mode, int sched) {
   const size_t n = g->m.size();
+  for (size_t i = 0; i < n; ++i) {
+    wdm_status s = start_state(g->m[i], g->st, sched);
+    if (s != WDM_OK) return group_fail(s, "wdm_group_step: " + g->m[i]->err);
+  }
   if (sched == GROUP_PERSISTENT) WDM_TRY(build_members(g, dt, mode, ver));
   if (sched == GROUP_STREAMS && g->fork.size() < n) {
     if (!g->ev_fork && cudaEventCreateWithFlags(&g->ev_fork, cudaEventDisableTiming) != cudaSuccess)
@@ -2257,7 +2355,10 @@ static wdm_status choose_schedule(wdm_group* g, const std::vector<double>& dt, c
     cudaMemcpyAsync(keep[2 * i], c->psi, sizeof(float2) * np, cudaMemcpyDeviceToDevice, g->st);
     cudaMemcpyAsync(keep[2 * i + 1], c->H, sizeof(float2) * nh, cudaMemcpyDeviceToDevice, g->st);
   }
-  // the tide-frame words of the last density pass belong to the saved state too
+  // the tide-frame words of the last density pass and the form of H belong to
+  // the saved state too
+  std::vector<int> h_y(n);
+  for (size_t i = 0; i < n; ++i) h_y[i] = g->m[i]->h_y;
   std::vector<std::vector<unsigned long long>> words(n);
   cudaStreamSynchronize(g->st);
   for (size_t i = 0; i < n; ++i)
@@ -2270,6 +2371,7 @@ static wdm_status choose_schedule(wdm_group* g, const std::vector<double>& dt, c
       wdm_ctx* c = g->m[i];
       cudaMemcpyAsync(c->psi, keep[2 * i], sizeof(float2) * c->ncell * c->d.batch, cudaMemcpyDeviceToDevice, g->st);
       cudaMemcpyAsync(c->H, keep[2 * i + 1], sizeof(float2) * c->nhalf * c->d.batch, cudaMemcpyDeviceToDevice, g->st);
+      c->h_y = h_y[i];
       if (!words[i].empty())
         cudaMemcpyAsync(c->centre, words[i].data(), sizeof(unsigned long long) * words[i].size(),
                         cudaMemcpyHostToDevice, g->st);
