@@ -1,7 +1,10 @@
 // Auxiliary kernels: density output, FP64 diagnostics reductions, CIC.
 #include "aux_kernels.cuh"
+#include "fft_factor.cuh"
 #include "tma.cuh"
 #include "wdm_math.cuh"
+
+#include <type_traits>
 
 namespace wdm {
 
@@ -89,231 +92,516 @@ cudaError_t launch_abs2(const float2* psi, float* out, long long n, cudaStream_t
   return cudaGetLastError();
 }
 
-// One block partial per (block, batch item): RED_FIELDS doubles.  The sums
-// restate src/visualization/runtime.jl:210-238 (interior cells, second-order
-// central differences) and src/simulation_main.jl:652 (total mass).
+// Diagnostics sums.  The sums restate src/visualization/runtime.jl:210-238
+// (interior cells, second-order central differences) and
+// src/simulation_main.jl:652 (total mass).
+//
+// A warp takes 32 neighbouring x of one row y and marches along z with the cell
+// below and the cell above it in registers: a cell's psi and |psi| are loaded and
+// formed once as the cell above, its x neighbours come from the neighbouring
+// lanes (the outer lanes load theirs), its y neighbours from memory (L1: the next
+// warps' rows).  A step's loads are issued one step ahead, behind an L2 prefetch.  That is four square roots per cell instead of seven.  Bound by
+// instruction issue (300 a cell, 63% of the slots: the per-cell terms, four IEEE
+// roots, a division, eleven compensated sums); 256^3 350 -> 210 us, with the
+// per-cell terms and the precision of the sums unchanged.
 constexpr int RED_THREADS = 128;
+constexpr int RED_CTAS = 5;   // resident blocks an SM
+constexpr int RED_AHEAD = 3;  // steps between a plane's L2 prefetch and its loads (without: 317 -> 297 us)
+// Cells along z of one march: long marches read the planes beside them less often,
+// short ones give every warp of the grid some work.
+static int red_depth(const RedGeom& g, int nblocks) {
+  int depth = 32;
+  auto tasks = [&] { return (long long)((g.nx + 31) / 32) * g.ny * ((g.nz + depth - 1) / depth); };
+  while (depth > 4 && tasks() < (long long)nblocks * (RED_THREADS / 32)) depth /= 2;
+  return depth;
+}
 
-// Per-thread running sum as an unevaluated float pair hi + lo (Knuth's
+// Two running sums side by side as unevaluated float pairs hi + lo (Knuth's
 // two-sum moves every rounding error of hi into lo).  A thread adds a few
-// hundred terms, so hi + lo carries the sum to about 2^-44 relative: FP64
+// hundred terms, so hi + lo carries each sum to about 2^-44 relative: FP64
 // accuracy for the totals without FP64 arithmetic per cell, which this GPU
 // runs at a small fraction of its FP32 rate.
-struct FAcc {
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(float v) {
-    const float s = hi + v;
-    const float bb = s - hi;
-    lo += (hi - (s - bb)) + (v - bb);
+struct FAcc2 {
+  float2 hi = {0.f, 0.f}, lo = {0.f, 0.f};
+  __device__ __forceinline__ void add(float u, float v) {
+    const float2 t = make_float2(u, v);
+    const float2 s = fx::add2(hi, t);
+    const float2 bb = fx::sub2(s, hi);
+    lo = fx::add2(lo, fx::add2(fx::sub2(hi, fx::sub2(s, bb)), fx::sub2(t, bb)));
     hi = s;
   }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ __forceinline__ double x() const { return (double)hi.x + (double)lo.x; }
+  __device__ __forceinline__ double y() const { return (double)hi.y + (double)lo.y; }
 };
 
-__global__ void __launch_bounds__(RED_THREADS)
-k_reduce(const float2* __restrict__ psi_all, const float* __restrict__ phi_all, RedGeom g,
+// One field's running value: sums, the largest |Phi|, the density maximum with the
+// first cell that holds it.
+struct RedTake {
+  int q;
+  double v, arg;
+  __device__ RedTake(int field, double v0, double arg0) : q(field), v(v0), arg(arg0) {}
+  __device__ __forceinline__ void take(double u, double ua) {
+    if (q == RED_MAX) {
+      if (u > v || (u == v && ua < arg)) {
+        v = u;
+        arg = ua;
+      }
+    } else if (q == RED_PHIMAX) {
+      v = fmax(v, u);
+    } else if (q != RED_ARG) {
+      v += u;
+    }
+  }
+  __device__ __forceinline__ void store(double* fields) const {
+    if (q == RED_ARG) return;  // comes with RED_MAX
+    fields[q] = v;
+    if (q == RED_MAX) fields[RED_ARG] = arg;
+  }
+};
+
+// One block partial per (block, batch item): RED_FIELDS doubles.
+__global__ void __launch_bounds__(RED_THREADS, RED_CTAS)
+k_reduce(const float2* __restrict__ psi_all, const float* __restrict__ phi_all, RedGeom g, int depth,
          double* __restrict__ partials) {
-  const long long nxy = (long long)g.nx * g.ny;
-  const long long n = nxy * g.nz;
+  const int nxy = g.nx * g.ny;  // an item has at most 512^3 cells
+  const long long n = (long long)nxy * g.nz;
   const float2* psi = psi_all + blockIdx.y * n;
   const float* phi = phi_all + blockIdx.y * n;
-  FAcc mass, mx, my, mz, wp, kk, q, px, py, pz;
+  FAcc2 m_w, mxy, mz_k, q_pz, pxy;  // (mass, W), (x, y), (z, K), (Q, pz), (px, py)
   float best_hi = -1.f, best_lo = 0.f, phimax = 0.f;
-  long long best_i = 0;
-  double sw = 0.0, swr = 0.0, swr2 = 0.0;  // one z-slice only: FP64 is cheap there
+  int best_i = 0;
   const float fi2dx = (float)(0.5 / g.dx), fi2dy = (float)(0.5 / g.dy), fi2dz = (float)(0.5 / g.dz);
   const float fx0 = (float)g.x0, fy0 = (float)g.y0, fz0 = (float)g.z0;
   const float fdx = (float)g.dx, fdy = (float)g.dy, fdz = (float)g.dz;
-  // rows (y, z) over the blocks, x over the threads: one index division per row
-  const long long nrows = (long long)g.ny * g.nz;
-  for (long long row = blockIdx.x; row < nrows; row += gridDim.x)
-  for (int x = threadIdx.x; x < g.nx; x += blockDim.x) {
-    const int z = (int)(row / g.ny);
-    const int y = (int)(row - (long long)z * g.ny);
-    const long long i = row * g.nx + x;
-    const float2 p = psi[i];
-    // rho = p.x^2 + p.y^2 exactly as (rs, rt): two-product of each square, two-sum of the pair
-    const float a = p.x * p.x, b = p.y * p.y;
-    const float ea = fmaf(p.x, p.x, -a), eb = fmaf(p.y, p.y, -b);
-    const float rs = a + b;
-    const float bb = rs - a;
-    const float rt = ((a - (rs - bb)) + (b - bb)) + (ea + eb);
-    mass.add(rs);
-    mass.lo += rt;
-    mx.add(rs * fmaf(fdx, (float)x, fx0));
-    my.add(rs * fmaf(fdy, (float)y, fy0));
-    mz.add(rs * fmaf(fdz, (float)z, fz0));
-    if (rs > best_hi || (rs == best_hi && rt > best_lo)) {
-      best_hi = rs;
-      best_lo = rt;
-      best_i = i;
-    }
-    const float ph = phi[i];
-    phimax = fmaxf(phimax, fabsf(ph));
-    if (z == g.zmid) {
-      const double rho = (double)rs + (double)rt;
-      const double fx = g.x0 + g.dx * x, fy = g.y0 + g.dy * y, fz = g.z0 + g.dz * z;
-      const double r2 = fx * fx + fy * fy + fz * fz;
-      sw += rho;
-      swr += rho * sqrt(r2);
-      swr2 += rho * r2;
-    }
-    if (x > 0 && x < g.nx - 1 && y > 0 && y < g.ny - 1 && z > 0 && z < g.nz - 1) {
+  auto mag = [](float2 v) { return sqrtf(fmaf(v.x, v.x, v.y * v.y)); };
+  const int lane = threadIdx.x & 31;
+  const int tiles = (g.nx + 31) / 32, depths = (g.nz + depth - 1) / depth;
+  const int tasks = tiles * g.ny * depths;  // neighbouring warps: neighbouring rows
+  for (int task = blockIdx.x * (RED_THREADS / 32) + (threadIdx.x >> 5); task < tasks; task += gridDim.x * (RED_THREADS / 32)) {
+    const int y = task % g.ny, td = task / g.ny, tx = td % tiles, z0 = (td / tiles) * depth;
+    const int z1 = z0 + depth < g.nz ? z0 + depth : g.nz;
+    const int x = tx * 32 + lane;
+    const bool in = x < g.nx;
+    const bool xy_inner = in && x > 0 && x < g.nx - 1 && y > 0 && y < g.ny - 1;
+    // the outer lanes' missing x neighbour
+    const bool edge = (lane == 0 && x > 0) || (lane == 31 && x < g.nx - 1);
+    const int i0 = z0 * nxy + y * g.nx + (in ? x : 0);
+    const float rx = fmaf(fdx, (float)x, fx0), ry = fmaf(fdy, (float)y, fy0);
+    const float2 zero = make_float2(0.f, 0.f);
+    const float2* ps = psi + i0;
+    const float* fs = phi + i0;
+    // a step's loads are issued one step ahead of their use
+    float2 n_zp = zero, n_e = zero, n_yp = zero, n_ym = zero;
+    float n_ph = 0.f;
+    auto load = [&](int z) {  // what step z reads; ps and fs point at its cell
+      n_zp = z + 1 < g.nz && in ? ps[nxy] : zero;
+      n_ph = in ? *fs : 0.f;
+      n_e = edge ? ps[lane == 0 ? -1 : 1] : zero;
+      n_yp = xy_inner ? ps[g.nx] : zero;
+      n_ym = xy_inner ? ps[-g.nx] : zero;
+    };
+    float2 zm = z0 > 0 && in ? ps[-nxy] : zero, p = in ? *ps : zero;
+    load(z0);
+    float mzm = mag(zm), mp = mag(p);
+    for (int z = z0; z < z1; ++z) {
+      const float2 zp = n_zp, e = n_e, yp = n_yp, ym = n_ym;
+      const float ph = n_ph;
+      ps += nxy;
+      fs += nxy;
+      if (z + 1 < z1) load(z + 1);
+      if (in && z + RED_AHEAD < z1) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(ps + RED_AHEAD * nxy));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(fs + (RED_AHEAD - 1) * nxy));
+      }
+      const float mzp = mag(zp);
+      const bool inner = xy_inner && z > 0 && z < g.nz - 1;
+      const float me = mag(e);
+      float2 xp, xm;
+      xp.x = __shfl_down_sync(0xffffffffu, p.x, 1);
+      xp.y = __shfl_down_sync(0xffffffffu, p.y, 1);
+      xm.x = __shfl_up_sync(0xffffffffu, p.x, 1);
+      xm.y = __shfl_up_sync(0xffffffffu, p.y, 1);
+      float mxp = __shfl_down_sync(0xffffffffu, mp, 1), mxm = __shfl_up_sync(0xffffffffu, mp, 1);
+      if (lane == 31) {
+        xp = e;
+        mxp = me;
+      }
+      if (lane == 0) {
+        xm = e;
+        mxm = me;
+      }
+      // rho = p.x^2 + p.y^2 as (rs, rt) to 2^-47: two-product of each square, two-sum of
+      // the pair, normalised for the comparison.  __fmul_rn: a product that the compiler
+      // fuses into one of the additions would no longer be the one whose rounding is ea.
+      const float a = __fmul_rn(p.x, p.x), b = __fmul_rn(p.y, p.y);
+      const float ea = fmaf(p.x, p.x, -a), eb = fmaf(p.y, p.y, -b);
+      const float r0 = a + b;
+      const float bb = r0 - a;
+      const float r1 = ((a - (r0 - bb)) + (b - bb)) + (ea + eb);
+      const float rs = r0 + r1, rt = r1 - (rs - r0);
+      if (in && rs >= best_hi) {
+        const int i = i0 + (z - z0) * nxy;
+        if (rs > best_hi || rt > best_lo || (rt == best_lo && i < best_i)) {
+          best_hi = rs;
+          best_lo = rt;
+          best_i = i;
+        }
+      }
+      phimax = fmaxf(phimax, fabsf(ph));
       // per-cell terms in FP32 (the reference forms them from its FP32 psi too)
-      wp.add(rs * ph);
-      const float2 xp = psi[i + 1], xm = psi[i - 1];
-      const float2 yp = psi[i + g.nx], ym = psi[i - g.nx];
-      const float2 zp = psi[i + nxy], zm = psi[i - nxy];
-      // rho v = Im(conj(psi) grad psi)
-      const float gxr = (xp.x - xm.x) * fi2dx, gxi = (xp.y - xm.y) * fi2dx;
-      const float gyr = (yp.x - ym.x) * fi2dy, gyi = (yp.y - ym.y) * fi2dy;
-      const float gzr = (zp.x - zm.x) * fi2dz, gzi = (zp.y - zm.y) * fi2dz;
-      const float jx = fmaf(p.x, gxi, -p.y * gxr);
-      const float jy = fmaf(p.x, gyi, -p.y * gyr);
-      const float jz = fmaf(p.x, gzi, -p.y * gzr);
-      px.add(jx);
-      py.add(jy);
-      pz.add(jz);
-      if (rs > 0.f) kk.add(fmaf(jx, jx, fmaf(jy, jy, jz * jz)) / rs);
-      auto mag = [](float2 v) { return sqrtf(fmaf(v.x, v.x, v.y * v.y)); };
-      const float ax = (mag(xp) - mag(xm)) * fi2dx;
-      const float ay = (mag(yp) - mag(ym)) * fi2dy;
-      const float az = (mag(zp) - mag(zm)) * fi2dz;
-      q.add(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+      float jx = 0.f, jy = 0.f, jz = 0.f, k = 0.f, q = 0.f;
+      if (inner) {
+        // rho v = Im(conj(psi) grad psi)
+        const float gxr = (xp.x - xm.x) * fi2dx, gxi = (xp.y - xm.y) * fi2dx;
+        const float gyr = (yp.x - ym.x) * fi2dy, gyi = (yp.y - ym.y) * fi2dy;
+        const float gzr = (zp.x - zm.x) * fi2dz, gzi = (zp.y - zm.y) * fi2dz;
+        jx = fmaf(p.x, gxi, -p.y * gxr);
+        jy = fmaf(p.x, gyi, -p.y * gyr);
+        jz = fmaf(p.x, gzi, -p.y * gzr);
+        if (rs > 0.f) k = fmaf(jx, jx, fmaf(jy, jy, jz * jz)) / rs;
+        const float ax = (mxp - mxm) * fi2dx;
+        const float ay = (mag(yp) - mag(ym)) * fi2dy;
+        const float az = (mzp - mzm) * fi2dz;
+        q = fmaf(ax, ax, fmaf(ay, ay, az * az));
+      }
+      m_w.add(rs, inner ? rs * ph : 0.f);
+      m_w.lo.x += rt;
+      mxy.add(rs * rx, rs * ry);
+      mz_k.add(rs * fmaf(fdz, (float)z, fz0), k);
+      q_pz.add(q, jz);
+      pxy.add(jx, jy);
+      zm = p;
+      mzm = mp;
+      p = zp;
+      mp = mzp;
     }
   }
-  double acc[RED_FIELDS];
-  acc[RED_MASS] = mass.value();
-  acc[RED_MAX] = best_hi < 0.f ? -1.0 : (double)best_hi + (double)best_lo;
-  acc[RED_ARG] = (double)best_i;
-  acc[RED_MX] = mx.value();
-  acc[RED_MY] = my.value();
-  acc[RED_MZ] = mz.value();
-  acc[RED_W] = wp.value();
-  acc[RED_K] = kk.value();
-  acc[RED_Q] = q.value();
-  acc[RED_PX] = px.value();
-  acc[RED_PY] = py.value();
-  acc[RED_PZ] = pz.value();
-  acc[RED_PHIMAX] = (double)phimax;
-  acc[RED_SW] = sw;
-  acc[RED_SWR] = swr;
-  acc[RED_SWR2] = swr2;
-  // block reduction (warp shuffles, then one warp over the warp results)
-  __shared__ double sh[RED_THREADS / 32][RED_FIELDS];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // one z-slice only: FP64 is cheap there
+  double sw = 0.0, swr = 0.0, swr2 = 0.0;
+  for (int c = blockIdx.x * RED_THREADS + threadIdx.x; c < nxy; c += gridDim.x * RED_THREADS) {
+    const int y = c / g.nx, x = c - y * g.nx;
+    const float2 p = psi[g.zmid * nxy + c];
+    const double rho = fma((double)p.x, (double)p.x, (double)p.y * p.y);
+    const double fx = g.x0 + g.dx * x, fy = g.y0 + g.dy * y, fz = g.z0 + g.dz * g.zmid;
+    const double r2 = fx * fx + fy * fy + fz * fz;
+    sw += rho;
+    swr += rho * sqrt(r2);
+    swr2 += rho * r2;
+  }
+  // The block's sums: eight threads a field, 16 values each (a shuffle tree over
+  // every field costs five times the FP64 additions, 22 us of the kernel)
+  static_assert(RED_FIELDS * 8 == RED_THREADS, "eight threads a field");
+  __shared__ double sh[RED_FIELDS][RED_THREADS + 2];
+  const int t = threadIdx.x;
+  sh[RED_MASS][t] = m_w.x();
+  sh[RED_MAX][t] = best_hi < 0.f ? -1.0 : (double)best_hi + (double)best_lo;
+  sh[RED_ARG][t] = (double)best_i;
+  sh[RED_MX][t] = mxy.x();
+  sh[RED_MY][t] = mxy.y();
+  sh[RED_MZ][t] = mz_k.x();
+  sh[RED_W][t] = m_w.y();
+  sh[RED_K][t] = mz_k.y();
+  sh[RED_Q][t] = q_pz.x();
+  sh[RED_PX][t] = pxy.x();
+  sh[RED_PY][t] = pxy.y();
+  sh[RED_PZ][t] = q_pz.y();
+  sh[RED_PHIMAX][t] = (double)phimax;
+  sh[RED_SW][t] = sw;
+  sh[RED_SWR][t] = swr;
+  sh[RED_SWR2][t] = swr2;
+  __syncthreads();
+  const int q = t >> 3, part = t & 7;
+  RedTake r(q, sh[q][part], sh[RED_ARG][part]);
+  for (int k = part + 8; k < RED_THREADS; k += 8) r.take(sh[q][k], sh[RED_ARG][k]);
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) {
+    const double u = __shfl_down_sync(0xffffffffu, r.v, off, 8), ua = __shfl_down_sync(0xffffffffu, r.arg, off, 8);
+    r.take(u, ua);
+  }
+  if (part == 0) r.store(partials + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * RED_FIELDS);
+}
+
+// The items' fields from their block partials: one warp, in a block of its own, per
+// field and item (FP64 runs at one a cycle and SM: 18 us with all fields on one SM).
+__global__ void __launch_bounds__(32)
+k_reduce_final(const double* __restrict__ partials, int nblocks, double* __restrict__ fields) {
+  const int lane = threadIdx.x, q = blockIdx.x;
+  if (q == RED_ARG) return;  // comes with RED_MAX
+  const double* o = partials + (long long)blockIdx.y * nblocks * RED_FIELDS;
+  RedTake r(q, q == RED_MAX ? -1.0 : 0.0, 0.0);
+  constexpr int U = 8;
+  for (int k0 = lane; k0 < nblocks; k0 += 32 * U) {
+    double u[U], ua[U];  // loads first: their latency is what the kernel takes
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const int k = k0 + 32 * j;
+      u[j] = k < nblocks ? o[k * RED_FIELDS + q] : q == RED_MAX ? -1.0 : 0.0;
+      ua[j] = k < nblocks ? o[k * RED_FIELDS + RED_ARG] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (k0 + 32 * j < nblocks) r.take(u[j], ua[j]);
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-    for (int q = 0; q < RED_FIELDS; ++q) {
-      const double o = __shfl_down_sync(0xffffffffu, acc[q], off);
-      if (q == RED_PHIMAX) acc[q] = fmax(acc[q], o);
-      if (red_is_max(q)) continue;
-      acc[q] += o;
-    }
-    const double om = __shfl_down_sync(0xffffffffu, acc[RED_MAX], off);
-    const double oa = __shfl_down_sync(0xffffffffu, acc[RED_ARG], off);
-    if (om > acc[RED_MAX] || (om == acc[RED_MAX] && oa < acc[RED_ARG])) {
-      acc[RED_MAX] = om;
-      acc[RED_ARG] = oa;
-    }
+    const double u = __shfl_down_sync(0xffffffffu, r.v, off), ua = __shfl_down_sync(0xffffffffu, r.arg, off);
+    r.take(u, ua);
   }
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < RED_FIELDS; ++q) sh[w][q] = acc[q];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r[RED_FIELDS];
-#pragma unroll
-    for (int q = 0; q < RED_FIELDS; ++q) r[q] = sh[0][q];
-    for (int k = 1; k < RED_THREADS / 32; ++k) {
-      for (int q = 0; q < RED_FIELDS; ++q)
-        if (!red_is_max(q)) r[q] += sh[k][q];
-      r[RED_PHIMAX] = fmax(r[RED_PHIMAX], sh[k][RED_PHIMAX]);
-      if (sh[k][RED_MAX] > r[RED_MAX] || (sh[k][RED_MAX] == r[RED_MAX] && sh[k][RED_ARG] < r[RED_ARG])) {
-        r[RED_MAX] = sh[k][RED_MAX];
-        r[RED_ARG] = sh[k][RED_ARG];
-      }
-    }
-    double* o = partials + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * RED_FIELDS;
-    for (int q = 0; q < RED_FIELDS; ++q) o[q] = r[q];
-  }
+  if (lane == 0) r.store(fields + blockIdx.y * RED_FIELDS);
 }
 
 cudaError_t launch_reduce(const float2* psi, const float* phi, const RedGeom& g, double* partials, int nblocks,
-                          int batch, cudaStream_t st) {
-  k_reduce<<<dim3(nblocks, batch), RED_THREADS, 0, st>>>(psi, phi, g, partials);
+                          int batch, double* fields, cudaStream_t st) {
+  k_reduce<<<dim3(nblocks, batch), RED_THREADS, 0, st>>>(psi, phi, g, red_depth(g, nblocks), partials);
+  k_reduce_final<<<dim3(RED_FIELDS, batch), 32, 0, st>>>(partials, nblocks, fields);
   return cudaGetLastError();
 }
 
-// Weights of the distances from the density maximum (the weighted quantiles of
-// src/simulation_main.jl:641-650), keyed by the squared distance in cells.  A
-// thread takes one offset (a, b, c) >= 0 and sums the up to eight cells at
-// (cx +- a, cy +- b, cz +- c) inside the grid, which share the key
+// ----------------------------------------------------------------------------
+// Lagrangian radii: the weighted quantiles of src/simulation_main.jl:641-650 of
+// the distance from the density maximum, on the device from the histogram to the
+// few numbers the quantiles need (RadiiOut): fetching the histogram and summing it
+// on the host took 0.3 ms of a 256^3 snapshot, beside 0.27 ms of kernels (now 0.1).
+// ----------------------------------------------------------------------------
+struct Centre {
+  int x, y, z;
+  __device__ Centre(const double* fields, int nx, int ny) {
+    const long long arg = (long long)fields[RED_ARG];
+    z = (int)(arg / ((long long)nx * ny));
+    const int rem = (int)(arg - (long long)z * nx * ny);
+    y = rem / nx;
+    x = rem - y * nx;
+  }
+};
+
+// Weights of the distances from the density maximum, keyed by the squared
+// distance in cells.  A thread takes one offset (a, b, c) >= 0 and sums the up to
+// eight cells at (cx +- a, cy +- b, cz +- c) inside the grid, which share the key
 // a^2 + b^2 + c^2, so a centred halo needs one atomic add per eight cells.
-__global__ void k_radii_hist(const float2* __restrict__ psi, int nx, int ny, int nz, int cx, int cy, int cz, int da,
-                             int db, int dc, double* __restrict__ wsum) {
-  const int nbc = db * dc;
-  for (int bc = blockIdx.x; bc < nbc; bc += gridDim.x)
-  for (int a = threadIdx.x; a < da; a += blockDim.x) {
-    const int c = bc / db;
-    const int b = bc - c * db;
+//
+// FP64 runs at one operation a cycle and SM, so two FP64 FMAs per cell took 145 us
+// at 256^3 (now 56).  The eight cells are summed in three FP32 words instead: squares as
+// exact pairs, every rounding of the leading sums kept by two-sums, roundings of
+// the third word alone lost (2^-70 of the sum), one rounding into FP64 at the end.
+// The squares' low words are exact for components from 2^-50 to 2^60 (and zero);
+// threads that meet another one sum in FP64.
+struct Sum3 {
+  float h = 0.f, m = 0.f, l = 0.f;
+  static __device__ __forceinline__ float two_sum(float& a, float b) {  // a += b, returns the rounding
+    const float s = a + b, t = s - a;
+    const float e = (a - (s - t)) + (b - t);
+    a = s;
+    return e;
+  }
+  __device__ __forceinline__ void add(float2 p) {
+    float s = __fmul_rn(p.x, p.x), e = fmaf(p.x, p.x, -s);
+    const float b = __fmul_rn(p.y, p.y), eb = fmaf(p.y, p.y, -b);
+    const float e1 = two_sum(s, b), e2 = two_sum(e, eb);
+    const float e3 = two_sum(h, s);
+    l += ((two_sum(m, e3) + two_sum(m, e1)) + two_sum(m, e)) + e2;
+  }
+  __device__ __forceinline__ double value() const { return (double)h + ((double)m + (double)l); }
+};
+
+__global__ void __launch_bounds__(256)
+k_radii_hist(const float2* __restrict__ psi, int nx, int ny, int nz, const double* __restrict__ fields,
+             double* __restrict__ wsum) {
+  const Centre o(fields, nx, ny);
+  const unsigned da = max(o.x, nx - 1 - o.x) + 1, db = max(o.y, ny - 1 - o.y) + 1, dc = max(o.z, nz - 1 - o.z) + 1;
+  const unsigned total = da * db * dc;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const unsigned bc = t / da;
+    const int a = (int)(t - bc * da), c = (int)(bc / db), b = (int)(bc - c * db);
+    float2 p[8];
+    bool exact = true;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int zz = k & 4 ? o.z - c : o.z + c, yy = k & 2 ? o.y - b : o.y + b, xx = k & 1 ? o.x - a : o.x + a;
+      const bool in = zz >= 0 && zz < nz && !(k & 4 && !c) && yy >= 0 && yy < ny && !(k & 2 && !b) && xx >= 0 &&
+                      xx < nx && !(k & 1 && !a);
+      p[k] = in ? psi[((long long)zz * ny + yy) * nx + xx] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float u = fabsf(p[k].x), v = fabsf(p[k].y);
+      exact = exact && (u == 0.f || (u >= 0x1p-50f && u < 0x1p60f)) && (v == 0.f || (v >= 0x1p-50f && v < 0x1p60f));
+    }
     double s = 0.0;
-    for (int sz = 0; sz < (c ? 2 : 1); ++sz) {
-      const int zz = sz ? cz - c : cz + c;
-      if (zz < 0 || zz >= nz) continue;
-      for (int sy = 0; sy < (b ? 2 : 1); ++sy) {
-        const int yy = sy ? cy - b : cy + b;
-        if (yy < 0 || yy >= ny) continue;
-        const long long row = ((long long)zz * ny + yy) * nx;
-        for (int sx = 0; sx < (a ? 2 : 1); ++sx) {
-          const int xx = sx ? cx - a : cx + a;
-          if (xx < 0 || xx >= nx) continue;
-          const float2 p = psi[row + xx];
-          s += (double)p.x * p.x + (double)p.y * p.y;
-        }
+    if (exact) {
+      Sum3 w;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w.add(p[k]);
+      if (w.h > 0.f) s = w.value();
+    } else {
+      for (int k = 0; k < 8; ++k) s = fma((double)p[k].x, (double)p[k].x, fma((double)p[k].y, (double)p[k].y, s));
+    }
+    if (s > 0.0) atomicAdd(&wsum[a * a + b * b + c * c], s);
+  }
+}
+
+// Per block of RADII_BLOCK keys: the sum of their weights and the last key with
+// weight (-1: none).
+constexpr int RADII_BLOCK = 1024;
+__global__ void __launch_bounds__(256)
+k_radii_blocks(const double* __restrict__ wsum, int nkeys, double* __restrict__ bsum, int* __restrict__ blast) {
+  const int base = blockIdx.x * RADII_BLOCK;
+  double s = 0.0;
+  int last = -1;
+#pragma unroll
+  for (int k = 0; k < RADII_BLOCK / 256; ++k) {
+    const int key = base + k * 256 + threadIdx.x;
+    const double w = key < nkeys ? wsum[key] : 0.0;
+    s += w;
+    if (w > 0.0) last = key;
+  }
+  __shared__ double ss[8];
+  __shared__ int sl[8];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    s += __shfl_down_sync(0xffffffffu, s, off);
+    last = max(last, __shfl_down_sync(0xffffffffu, last, off));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    ss[threadIdx.x >> 5] = s;
+    sl[threadIdx.x >> 5] = last;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) {
+      s += ss[k];
+      last = max(last, sl[k]);
+    }
+    bsum[blockIdx.x] = s;
+    blast[blockIdx.x] = last;
+  }
+}
+
+// Inclusive sums over a block of RADII_BLOCK = 32 x 32 threads: one warp adds 32
+// values a lane (a scan by shuffles in every warp does 5 FP64 additions a value,
+// at one a cycle: 15 us for the kernel).  `sh`: 33 x 32 + 32 words.
+__device__ double radii_scan(double v, double* sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* off = sh + 33 * 32;
+  __syncthreads();  // sh may still be read from the scan before
+  sh[33 * w + lane] = v;
+  __syncthreads();
+  if (w == 0) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) sh[33 * lane + k] = s += sh[33 * lane + k];
+    double t = s;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const double u = __shfl_up_sync(0xffffffffu, t, d);
+      if (lane >= d) t += u;
+    }
+    off[lane] = t;
+  }
+  __syncthreads();
+  return w ? sh[33 * w + lane] + off[w - 1] : sh[lane];
+}
+
+// The groups the quantiles fall in, one block a quantile: h = p (S - w_1) + w_1
+// (w_1: the weight at distance 0), the first key whose cumulative weight exceeds h,
+// the cumulative weight and the key with weight before it.
+__global__ void __launch_bounds__(RADII_BLOCK)
+k_radii_find(const double* __restrict__ wsum, int nkeys, const double* __restrict__ bsum,
+             const int* __restrict__ blast, int nblocks, RadiiOut* __restrict__ out) {
+  __shared__ double scan[33 * 32 + 32], before;
+  __shared__ int last[RADII_BLOCK], block, first, prev;
+  const int t = threadIdx.x, q = blockIdx.x;
+  const double w1 = wsum[0];
+  const double own = t < nblocks ? bsum[t] : 0.0;
+  last[t] = t < nblocks ? blast[t] : -1;
+  if (t == 0) {
+    block = nblocks;
+    first = RADII_BLOCK;
+    prev = -1;
+  }
+  const double incl = radii_scan(own, scan);
+  const double total = scan[33 * 32 + 31];
+  const double h = radii_p(q) * (total - w1) + w1;
+  if (own > 0.0 && incl > h) atomicMin(&block, t);
+  __syncthreads();
+  const int blk = block;
+  if (t == 0) {
+    out->wmin[q] = ~0ull;
+    if (q == 0) {
+      int k = nblocks - 1;
+      while (k >= 0 && last[k] < 0) --k;
+      out->last = k >= 0 ? last[k] : -1;
+      out->total = total;
+      out->w1 = w1;
+    }
+    if (blk == nblocks) out->key[q] = -1;
+  }
+  if (blk == nblocks) return;
+  if (t == blk) before = incl - own;
+  const int key = blk * RADII_BLOCK + t;
+  const double w = key < nkeys ? wsum[key] : 0.0;
+  const double in_block = radii_scan(w, scan);
+  const double cum = before + in_block;
+  // the block's sum and the cumulative sum round differently: with no key past h its last one is meant
+  if (w > 0.0 && (cum > h || key == last[blk])) atomicMin(&first, t);
+  __syncthreads();
+  if (w > 0.0 && t < first) atomicMax(&prev, t);
+  __syncthreads();
+  if (t == first) {
+    int k = blk - 1;
+    while (k >= 0 && last[k] < 0) --k;
+    out->key[q] = key;
+    out->prev[q] = prev >= 0 ? blk * RADII_BLOCK + prev : k >= 0 ? last[k] : -1;
+    out->before[q] = cum - w;
+  }
+}
+
+// Smallest nonzero weight (bits of a positive double) among the cells of each
+// group the quantiles fall in: a row (y, z) holds at most the two cells cx +- r of
+// a key, r^2 = key - dy^2 - dz^2.
+__global__ void __launch_bounds__(256)
+k_radii_min(const float2* __restrict__ psi, int nx, int ny, int nz, const double* __restrict__ fields,
+            RadiiOut* __restrict__ out) {
+  const Centre o(fields, nx, ny);
+  const int nrows = ny * nz;
+  int key[RADII_QUANTILES];
+#pragma unroll
+  for (int q = 0; q < RADII_QUANTILES; ++q) key[q] = out->key[q];
+  for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < nrows; row += gridDim.x * blockDim.x) {
+    const int z = row / ny, y = row - z * ny;
+    const int d = (y - o.y) * (y - o.y) + (z - o.z) * (z - o.z);
+#pragma unroll
+    for (int q = 0; q < RADII_QUANTILES; ++q) {
+      const int rem = key[q] - d;
+      if (rem < 0) continue;
+      int r = (int)sqrtf((float)rem);
+      while (r * r > rem) --r;
+      while ((r + 1) * (r + 1) <= rem) ++r;
+      if (r * r != rem) continue;
+      for (int side = 0; side < (r ? 2 : 1); ++side) {
+        const int x = side ? o.x - r : o.x + r;
+        if (x < 0 || x >= nx) continue;
+        const float2 p = psi[(long long)row * nx + x];
+        const double rho = (double)p.x * p.x + (double)p.y * p.y;
+        if (rho > 0.0) atomicMin(&out->wmin[q], (unsigned long long)__double_as_longlong(rho));
       }
     }
-    if (s > 0.0) atomicAdd(&wsum[(long long)a * a + (long long)b * b + (long long)c * c], s);
   }
 }
 
-cudaError_t launch_radii_hist(const float2* psi, int nx, int ny, int nz, int cx, int cy, int cz, double* wsum,
-                              cudaStream_t st) {
-  const int da = (cx > nx - 1 - cx ? cx : nx - 1 - cx) + 1;
-  const int db = (cy > ny - 1 - cy ? cy : ny - 1 - cy) + 1;
-  const int dc = (cz > nz - 1 - cz ? cz : nz - 1 - cz) + 1;
-  const int rows = db * dc;
-  k_radii_hist<<<(unsigned)(rows < 152 * 32 ? rows : 152 * 32), 128, 0, st>>>(psi, nx, ny, nz, cx, cy, cz, da, db, dc,
-                                                                              wsum);
-  return cudaGetLastError();
-}
+int radii_blocks(long long nkeys) { return (int)((nkeys + RADII_BLOCK - 1) / RADII_BLOCK); }
 
-// Smallest nonzero weight (bits of a positive double) among the cells whose
-// key is one of keys.k[0..n): the few groups the quantiles fall in.
-__global__ void k_radii_min(const float2* __restrict__ psi, int nx, int ny, int nz, int cx, int cy, int cz,
-                            RadiiKeys keys, unsigned long long* __restrict__ wmin) {
-  const int nrows = ny * nz;
-  for (int row = blockIdx.x; row < nrows; row += gridDim.x)
-  for (int x = threadIdx.x; x < nx; x += blockDim.x) {
-    const int z = row / ny;
-    const int y = row - z * ny;
-    const long long i = (long long)row * nx + x;
-    const long long ddx = x - cx, ddy = y - cy, ddz = z - cz;
-    const long long key = ddx * ddx + ddy * ddy + ddz * ddz;
-    for (int j = 0; j < keys.n; ++j)
-      if (key == keys.k[j]) {
-        const float2 p = psi[i];
-        const double rho = (double)p.x * p.x + (double)p.y * p.y;
-        if (rho > 0.0) atomicMin(&wmin[j], (unsigned long long)__double_as_longlong(rho));
-      }
-  }
-}
-
-cudaError_t launch_radii_min(const float2* psi, int nx, int ny, int nz, int cx, int cy, int cz, const RadiiKeys& keys,
-                             unsigned long long* wmin, cudaStream_t st) {
-  const int rows = ny * nz;
-  k_radii_min<<<(unsigned)(rows < 152 * 32 ? rows : 152 * 32), 128, 0, st>>>(psi, nx, ny, nz, cx, cy, cz, keys, wmin);
+cudaError_t launch_radii(const float2* psi, int nx, int ny, int nz, const double* fields, double* wsum, long long nkeys,
+                         double* bsum, int* blast, RadiiOut* out, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(wsum, 0, sizeof(double) * nkeys, st);
+  if (e != cudaSuccess) return e;
+  const long long cells = (long long)nx * ny * nz;
+  const long long want = (cells + 255) / 256;  // the centre is known on the device only
+  k_radii_hist<<<(unsigned)(want < 152 * 8 ? want : 152 * 8), 256, 0, st>>>(psi, nx, ny, nz, fields, wsum);
+  const int nb = radii_blocks(nkeys);
+  k_radii_blocks<<<nb, 256, 0, st>>>(wsum, (int)nkeys, bsum, blast);
+  k_radii_find<<<RADII_QUANTILES, RADII_BLOCK, 0, st>>>(wsum, (int)nkeys, bsum, blast, nb, out);
+  const int rows = (ny * nz + 255) / 256;
+  k_radii_min<<<rows < 152 * 4 ? rows : 152 * 4, 256, 0, st>>>(psi, nx, ny, nz, fields, out);
   return cudaGetLastError();
 }
 
@@ -380,15 +668,26 @@ template <bool COMPLEX>
 __global__ void k_block_sum(const void* __restrict__ data, long long n, double* __restrict__ sums) {
   // per-thread FP32 partial sums (the shift only needs to be near the mean:
   // any value is exact), FP64 from the warp reduction on
+  // eight loads in flight per thread (one at a time left DRAM at half its rate:
+  // 256^3 38 us), added in the order of a plain loop
+  using T = std::conditional_t<COMPLEX, float2, float>;
+  constexpr int U = 8;
+  const T* p = static_cast<const T*>(data) + blockIdx.y * n;
+  const long long step = (long long)gridDim.x * blockDim.x;
   float accf = 0.f;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if constexpr (COMPLEX) {
-      const float2 v = static_cast<const float2*>(data)[blockIdx.y * n + i];
-      accf = fmaf(v.x, v.x, fmaf(v.y, v.y, accf));
-    } else {
-      accf += static_cast<const float*>(data)[blockIdx.y * n + i];
-    }
+  auto add = [&](T v) {
+    if constexpr (COMPLEX) accf = fmaf(v.x, v.x, fmaf(v.y, v.y, accf));
+    else accf += v;
+  };
+  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (; i + (U - 1) * step < n; i += U * step) {
+    T v[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) v[k] = p[i + k * step];
+#pragma unroll
+    for (int k = 0; k < U; ++k) add(v[k]);
   }
+  for (; i < n; i += step) add(p[i]);
   double acc = accf;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);

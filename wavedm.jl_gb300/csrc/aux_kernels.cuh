@@ -41,19 +41,27 @@ struct RedGeom {
   int zmid;  // z index of the slice the RED_SW* sums cover
 };
 
-// Lagrangian radii: per squared cell distance key = di^2 + dj^2 + dk^2 from
-// cell (cx, cy, cz), the FP64 sum of rho over the cells at that distance;
-// then, for up to RADII_KEYS keys, the smallest nonzero rho (as the bits of a
-// positive double) over their cells.
-constexpr int RADII_KEYS = 16;
-struct RadiiKeys {
-  long long k[RADII_KEYS];
-  int n;
+// Lagrangian radii about the density maximum (RED_ARG of `fields`): per squared
+// cell distance key = di^2 + dj^2 + dk^2 the FP64 sum of rho over the cells at
+// that distance (wsum, nkeys words), and what the nine quantiles read of it.
+// bsum and blast: radii_blocks(nkeys) words.
+constexpr int RADII_QUANTILES = 9;
+__host__ __device__ constexpr double radii_p(int q) {
+  constexpr double p[RADII_QUANTILES] = {0.1, 0.2, 0.3, 0.4, 0.5, 0.6, 0.7, 0.8, 0.9};
+  return p[q];
+}
+struct RadiiOut {
+  double total;                    // sum of all weights
+  double w1;                       // the weight at distance 0
+  double before[RADII_QUANTILES];  // cumulative weight before the quantile's group
+  unsigned long long wmin[RADII_QUANTILES];  // bits of the group's smallest weight
+  int key[RADII_QUANTILES];        // the group's key (-1: past the last one)
+  int prev[RADII_QUANTILES];       // the key with weight before it (-1: none)
+  int last;                        // the last key with weight (-1: none)
 };
-cudaError_t launch_radii_hist(const float2* psi, int nx, int ny, int nz, int cx, int cy, int cz, double* wsum,
-                              cudaStream_t st);
-cudaError_t launch_radii_min(const float2* psi, int nx, int ny, int nz, int cx, int cy, int cz, const RadiiKeys& keys,
-                             unsigned long long* wmin, cudaStream_t st);
+int radii_blocks(long long nkeys);
+cudaError_t launch_radii(const float2* psi, int nx, int ny, int nz, const double* fields, double* wsum, long long nkeys,
+                         double* bsum, int* blast, RadiiOut* out, cudaStream_t st);
 
 cudaError_t launch_abs2(const float2* psi, float* out, long long n, cudaStream_t st);
 // Adjoint seed of L = sum (|psi|^2 - rho_t)^2 dV: lam = 4 (|psi|^2 - rho_t) psi dV,
@@ -67,8 +75,9 @@ cudaError_t launch_sincos_half(const float* h, float* out, long long n, cudaStre
 // shift[b] = mean over item b of |data|^2 (complex_in) or of data (float), + add
 cudaError_t launch_mean_shift(const void* data, bool complex_in, long long n, int batch, double* sums, float* shift,
                               double add, cudaStream_t st);
+// fields[b]: the RED_FIELDS of batch item b (partials: nblocks x RED_FIELDS per item)
 cudaError_t launch_reduce(const float2* psi, const float* phi, const RedGeom& g, double* partials, int nblocks,
-                          int batch, cudaStream_t st);
+                          int batch, double* fields, cudaStream_t st);
 // CIC deposit of the particles into rho, which must be zero; rows (ny * nz
 // ints, may be null) flags the x rows that hold deposited mass.  The deposit
 // of static particles is kept: every density pass reads its flagged rows, and

@@ -222,9 +222,8 @@ struct wdm_ctx {
   // potential once, before the loop), so the deposit is made once per
   // particle set and every density pass reads it.
   int rb_ready = 0;
-  // diagnostics: radii histogram and minimum words (allocated on first use)
+  // diagnostics: radii histogram and its block sums (allocated on first use)
   double* diag_wsum = nullptr;
-  unsigned long long* diag_wmin = nullptr;
   long long version = 0;            // bumped by every set_* call that a captured graph bakes in
   struct wdm_group* self_group = nullptr;  // single-member group of wdm_step_graph
   Profiler prof;
@@ -833,6 +832,29 @@ static wdm_status copy_out(wdm_ctx* c, void* dst, const void* src, size_t bytes,
   return WDM_OK;
 }
 
+// The RED_* fields of the batch items, then their RadiiOut, in one buffer behind
+// the block partials: one copy brings a call's results to the host.
+static double* red_fields(const wdm_ctx* c) {
+  return c->red + (size_t)c->red_blocks * RED_FIELDS * c->d.batch;
+}
+static RadiiOut* red_radii(const wdm_ctx* c) { return (RadiiOut*)(red_fields(c) + (size_t)RED_FIELDS * c->d.batch); }
+static size_t red_size(const wdm_ctx* c) {  // doubles
+  return (size_t)c->d.batch * (((size_t)c->red_blocks + 1) * RED_FIELDS + sizeof(RadiiOut) / sizeof(double));
+}
+
+// The kernel that makes an output writes it to the caller's buffer itself, if
+// that is this device's memory (256^3: 20 us of copy less); `scratch` and copy_out
+// serve every other pointer.
+static float* output_buffer(const wdm_ctx* c, float* out, int where, float* scratch) {
+  cudaPointerAttributes a{}, own{};
+  if (where != WDM_DEVICE || !out || (uintptr_t)out % 16) return scratch;
+  if (cudaPointerGetAttributes(&a, out) != cudaSuccess || cudaPointerGetAttributes(&own, c->psi) != cudaSuccess) {
+    cudaGetLastError();
+    return scratch;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == own.device ? out : scratch;
+}
+
 static wdm_status ensure_scratch(wdm_ctx* c) {
   if (!c->scratch_f) WDM_TRY(dalloc(c, &c->scratch_f, (size_t)c->ncell * c->d.batch));
   if (!c->scratch_h) WDM_TRY(dalloc(c, &c->scratch_h, (size_t)c->nhalf * c->d.batch));
@@ -870,7 +892,7 @@ wdm_status wdm_destroy(wdm_ctx* c) {
                   c->scratch_h, c->red, c->sums, c->shift, c->shift_in};
   for (void* p : bufs)
     if (p) cudaFree(p);
-  void* adj[] = {c->ftx, c->fty, c->ftz, c->lam, c->Hmu, c->rho_t, c->D6, c->adj_acc, c->diag_wsum, c->diag_wmin, c->centre, c->frame};
+  void* adj[] = {c->ftx, c->fty, c->ftz, c->lam, c->Hmu, c->rho_t, c->D6, c->adj_acc, c->diag_wsum, c->centre, c->frame};
   for (void* p : adj)
     if (p) cudaFree(p);
   for (auto* v : {&c->ck_psi, &c->ck_H, &c->slot_psi, &c->slot_H, &c->slot2_psi, &c->slot2_H})
@@ -1114,8 +1136,8 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
     cuda_fail(c, e, "memset flag");
     return bail(WDM_ERR_CUDA);
   }
-  c->red_blocks = 4 * 152;
-  if ((s = dalloc(c, &c->red, B * c->red_blocks * RED_FIELDS)) != WDM_OK) return bail(s);
+  c->red_blocks = 5 * 152;  // k_reduce's resident blocks
+  if ((s = dalloc(c, &c->red, red_size(c))) != WDM_OK) return bail(s);
   if ((s = dalloc(c, &c->sums, B)) != WDM_OK) return bail(s);
   if ((s = dalloc(c, &c->shift, B)) != WDM_OK) return bail(s);
   if ((s = dalloc(c, &c->shift_in, B)) != WDM_OK) return bail(s);
@@ -1154,13 +1176,18 @@ wdm_status wdm_get_psi(wdm_ctx* c, void* psi, int32_t where) {
 wdm_status wdm_get_rho(wdm_ctx* c, float* rho, int32_t where) {
   WDM_TRY(need_psi(c));
   WDM_TRY(ensure_scratch(c));
-  cudaError_t e = launch_abs2(c->psi, c->scratch_f, c->ncell * c->d.batch, c->st);
+  float* dst = output_buffer(c, rho, where, c->scratch_f);
+  cudaError_t e = launch_abs2(c->psi, dst, c->ncell * c->d.batch, c->st);
   if (e != cudaSuccess) return cuda_fail(c, e, "abs2");
-  return copy_out(c, rho, c->scratch_f, sizeof(float) * c->ncell * c->d.batch, where);
+  if (dst != rho) return copy_out(c, rho, dst, sizeof(float) * c->ncell * c->d.batch, where);
+  WDM_CU(c, cudaStreamSynchronize(c->st));
+  return WDM_OK;
 }
 
-static wdm_status phi_real(wdm_ctx* c) {
+// Phi in real space, in `out` (the scratch field by default)
+static wdm_status phi_real(wdm_ctx* c, float* out = nullptr) {
   WDM_TRY(ensure_scratch(c));
+  float* dst = out ? out : c->scratch_f;
   if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, 0.0));
   // a y-spectral H stays as it is (the next kick and captured graphs start from it)
   float2* H = c->H;
@@ -1174,7 +1201,7 @@ static wdm_status phi_real(wdm_ctx* c) {
     H = c->scratch_h;
   }
   cudaError_t e = run_pass(c, P_PHI_OUT, [&] {
-    return c->fx->c2r(H, c->scratch_f, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
+    return c->fx->c2r(H, dst, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
   });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_c2r");
   return WDM_OK;
@@ -1182,8 +1209,12 @@ static wdm_status phi_real(wdm_ctx* c) {
 
 wdm_status wdm_get_phi(wdm_ctx* c, float* phi, int32_t where) {
   WDM_TRY(need_psi(c));
-  WDM_TRY(phi_real(c));
-  return copy_out(c, phi, c->scratch_f, sizeof(float) * c->ncell * c->d.batch, where);
+  WDM_TRY(ensure_scratch(c));
+  float* dst = output_buffer(c, phi, where, c->scratch_f);
+  WDM_TRY(phi_real(c, dst));
+  if (dst != phi) return copy_out(c, phi, dst, sizeof(float) * c->ncell * c->d.batch, where);
+  WDM_CU(c, cudaStreamSynchronize(c->st));
+  return WDM_OK;
 }
 
 wdm_status wdm_set_static_potential(wdm_ctx* c, const float* V, int32_t where) {
@@ -1421,9 +1452,8 @@ wdm_status wdm_fft3d(wdm_ctx* c, void* data, int32_t dir) {
   return WDM_OK;
 }
 
-// The per-item FP64 reduction of psi and Phi (k_reduce), block partials
-// combined on the host: r[b] holds the RED_* fields of batch item b.
-static wdm_status reduce_items(wdm_ctx* c, std::vector<std::array<double, RED_FIELDS>>& r) {
+// The per-item FP64 reduction of psi and Phi into red_fields (queued).
+static wdm_status reduce_items(wdm_ctx* c) {
   WDM_TRY(phi_real(c));
   RedGeom g;
   g.nx = c->d.nx;
@@ -1436,32 +1466,13 @@ static wdm_status reduce_items(wdm_ctx* c, std::vector<std::array<double, RED_FI
   g.y0 = c->y0;
   g.z0 = c->z0;
   g.zmid = c->d.nz / 2 - 1 > 0 ? c->d.nz / 2 - 1 : 0;  // the slice div(end, 2) of a 1-based z axis
-  cudaError_t e = launch_reduce(c->psi, c->scratch_f, g, c->red, c->red_blocks, c->d.batch, c->st);
+  cudaError_t e = launch_reduce(c->psi, c->scratch_f, g, c->red, c->red_blocks, c->d.batch, red_fields(c), c->st);
   if (e != cudaSuccess) return cuda_fail(c, e, "reduce");
-  std::vector<double> h((size_t)c->red_blocks * RED_FIELDS * c->d.batch);
-  WDM_CU(c, cudaMemcpyAsync(h.data(), c->red, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  WDM_CU(c, cudaStreamSynchronize(c->st));
-  r.assign((size_t)c->d.batch, {});
-  for (int b = 0; b < c->d.batch; ++b) {
-    std::array<double, RED_FIELDS>& acc = r[(size_t)b];
-    acc.fill(0.0);
-    acc[RED_MAX] = -1.0;
-    for (int k = 0; k < c->red_blocks; ++k) {
-      const double* p = &h[((size_t)b * c->red_blocks + k) * RED_FIELDS];
-      for (int q = 0; q < RED_FIELDS; ++q)
-        if (!red_is_max(q)) acc[q] += p[q];
-      acc[RED_PHIMAX] = std::max(acc[RED_PHIMAX], p[RED_PHIMAX]);
-      if (p[RED_MAX] > acc[RED_MAX] || (p[RED_MAX] == acc[RED_MAX] && p[RED_ARG] < acc[RED_ARG])) {
-        acc[RED_MAX] = p[RED_MAX];
-        acc[RED_ARG] = p[RED_ARG];
-      }
-    }
-  }
   return WDM_OK;
 }
 
 // The ten fields of wdm_reduce from one item's RED_* sums.
-static void reduce_fields(const wdm_ctx* c, const std::array<double, RED_FIELDS>& acc, double* o) {
+static void reduce_fields(const wdm_ctx* c, const double* acc, double* o) {
   const double dV = c->dx * c->dy * c->dz;
   const double m = acc[RED_MASS];
   o[0] = m * dV;
@@ -1482,9 +1493,11 @@ static void reduce_fields(const wdm_ctx* c, const std::array<double, RED_FIELDS>
 wdm_status wdm_reduce(wdm_ctx* c, double* out) {
   WDM_TRY(need_psi(c));
   if (!out) return fail(c, WDM_ERR_INVALID, "null output");
-  std::vector<std::array<double, RED_FIELDS>> r;
-  WDM_TRY(reduce_items(c, r));
-  for (int b = 0; b < c->d.batch; ++b) reduce_fields(c, r[(size_t)b], out + 10 * b);
+  WDM_TRY(reduce_items(c));
+  std::vector<double> r((size_t)RED_FIELDS * c->d.batch);
+  WDM_CU(c, cudaMemcpyAsync(r.data(), red_fields(c), r.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  WDM_CU(c, cudaStreamSynchronize(c->st));
+  for (int b = 0; b < c->d.batch; ++b) reduce_fields(c, &r[(size_t)RED_FIELDS * b], out + 10 * b);
   return WDM_OK;
 }
 
@@ -1554,29 +1567,58 @@ wdm_status wdm_weighted_quantiles_grouped(const double* value, const double* wsu
   return WDM_OK;
 }
 
+// The quantiles of an item's distances from its maximum: the rule of
+// grouped_quantiles on the groups that the device found.
+static void radii_quantiles(const RadiiOut& r, double dx, double* out) {
+  auto value = [dx](int key) { return dx * std::sqrt((double)key); };
+  for (int q = 0; q < RADII_QUANTILES; ++q) {
+    if (r.last < 0) {
+      out[q] = NAN;
+      continue;
+    }
+    if (r.key[q] < 0) {
+      out[q] = value(r.last);
+      continue;
+    }
+    const double h = radii_p(q) * (r.total - r.w1) + r.w1;
+    const double v = value(r.key[q]), vprev = r.prev[q] >= 0 ? value(r.prev[q]) : 0.0;
+    double m;
+    std::memcpy(&m, &r.wmin[q], sizeof(m));
+    out[q] = h < r.before[q] + m ? vprev + (h - r.before[q]) / m * (v - vprev) : v;
+  }
+}
+
 wdm_status wdm_diagnostics(wdm_ctx* c, double* out) {
   WDM_TRY(need_psi(c));
   if (!out) return fail(c, WDM_ERR_INVALID, "null output");
-  std::vector<std::array<double, RED_FIELDS>> r;
-  WDM_TRY(reduce_items(c, r));
-  const int nx = c->d.nx, ny = c->d.ny, nz = c->d.nz;
+  WDM_TRY(reduce_items(c));
+  const int nx = c->d.nx, ny = c->d.ny, nz = c->d.nz, B = c->d.batch;
   // the radii need equal spacings: squared distances are then dx^2 times an integer key
   const double tol = 1e-12 * c->dx;
   const bool cubic = std::fabs(c->dx - c->dy) <= tol && std::fabs(c->dx - c->dz) <= tol;
-  const int64_t nkeys = (int64_t)(nx - 1) * (nx - 1) + (int64_t)(ny - 1) * (ny - 1) + (int64_t)(nz - 1) * (nz - 1) + 1;
-  std::vector<double> hs;
+  const double* fields = red_fields(c);
   if (cubic) {
-    // the histogram (nkeys doubles) and the minimum words live with the context
-    if (!c->diag_wsum) WDM_TRY(dalloc(c, &c->diag_wsum, (size_t)nkeys));
-    if (!c->diag_wmin) WDM_TRY(dalloc(c, &c->diag_wmin, (size_t)RADII_KEYS));
-    hs.resize((size_t)nkeys);
+    const int64_t nkeys =
+        (int64_t)(nx - 1) * (nx - 1) + (int64_t)(ny - 1) * (ny - 1) + (int64_t)(nz - 1) * (nz - 1) + 1;
+    const size_t nblocks = (size_t)radii_blocks(nkeys);
+    // the histogram and its block sums live with the context; the items take turns
+    if (!c->diag_wsum) WDM_TRY(dalloc(c, &c->diag_wsum, (size_t)nkeys + 2 * nblocks));
+    double* bsum = c->diag_wsum + nkeys;
+    int* blast = (int*)(bsum + nblocks);
+    for (int b = 0; b < B; ++b) {
+      cudaError_t e = launch_radii(c->psi + (size_t)b * c->ncell, nx, ny, nz, fields + (size_t)RED_FIELDS * b,
+                                   c->diag_wsum, nkeys, bsum, blast, red_radii(c) + b, c->st);
+      if (e != cudaSuccess) return cuda_fail(c, e, "diagnostics histogram");
+      c->launch_count += 4;
+    }
   }
-  double* wsum = c->diag_wsum;
-  unsigned long long* wmin = c->diag_wmin;
-  static const double P[9] = {0.1, 0.2, 0.3, 0.4, 0.5, 0.6, 0.7, 0.8, 0.9};
-  wdm_status s = WDM_OK;
-  for (int b = 0; b < c->d.batch && s == WDM_OK; ++b) {
-    const auto& acc = r[(size_t)b];
+  std::vector<double> host((size_t)B * (RED_FIELDS + sizeof(RadiiOut) / sizeof(double)));
+  const size_t bytes = (cubic ? host.size() : (size_t)B * RED_FIELDS) * sizeof(double);
+  WDM_CU(c, cudaMemcpyAsync(host.data(), fields, bytes, cudaMemcpyDeviceToHost, c->st));
+  WDM_CU(c, cudaStreamSynchronize(c->st));
+  const RadiiOut* radii = (const RadiiOut*)&host[(size_t)B * RED_FIELDS];
+  for (int b = 0; b < B; ++b) {
+    const double* acc = &host[(size_t)RED_FIELDS * b];
     double* o = out + (size_t)WDM_DIAG_FIELDS * b;
     reduce_fields(c, acc, o);
     const double dV = c->dx * c->dy * c->dz;
@@ -1595,55 +1637,11 @@ wdm_status wdm_diagnostics(wdm_ctx* c, double* out) {
     } else {
       o[18] = NAN;
     }
-    if (!cubic) {
-      for (int i = 0; i < 9; ++i) o[19 + i] = NAN;
-      continue;
-    }
-    const long long arg = (long long)acc[RED_ARG];
-    const int cz = (int)(arg / ((long long)nx * ny)), rem = (int)(arg - (long long)cz * nx * ny);
-    const int cy = rem / nx, cx = rem - cy * nx;
-    // pass 1: the weight of every distance
-    cudaError_t e = cudaMemsetAsync(wsum, 0, sizeof(double) * nkeys, c->st);
-    const float2* pb = c->psi + (size_t)b * c->ncell;
-    if (e == cudaSuccess) e = launch_radii_hist(pb, nx, ny, nz, cx, cy, cz, wsum, c->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hs.data(), wsum, sizeof(double) * nkeys, cudaMemcpyDeviceToHost, c->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-    // pass 2: the smallest element weight of the distance 0 (w_1) and of the
-    // groups the quantiles fall in, the only ones the quantile reads
-    RadiiKeys keys{};
-    keys.k[keys.n++] = 0;
-    const GroupCum gc(hs.data(), e == cudaSuccess ? nkeys : 0);
-    if (!gc.idx.empty())
-      for (int i = 0; i < 9; ++i) {
-        const size_t k = gc.find(gc.h(P[i], acc[RED_MAX]));  // w_1 is the maximum's weight
-        if (k >= gc.idx.size()) continue;
-        const long long key = gc.idx[k];
-        if (std::find(keys.k, keys.k + keys.n, key) == keys.k + keys.n && keys.n < RADII_KEYS) keys.k[keys.n++] = key;
-      }
-    unsigned long long m[RADII_KEYS];
-    if (e == cudaSuccess) e = cudaMemsetAsync(wmin, 0xff, sizeof(unsigned long long) * RADII_KEYS, c->st);
-    if (e == cudaSuccess) e = launch_radii_min(pb, nx, ny, nz, cx, cy, cz, keys, wmin, c->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(m, wmin, sizeof(m), cudaMemcpyDeviceToHost, c->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-    if (e != cudaSuccess) {
-      s = cuda_fail(c, e, "diagnostics histogram");
-      break;
-    }
-    c->launch_count += 2;
-    const double dx = c->dx;
-    auto value = [dx](int64_t g) { return dx * std::sqrt((double)g); };
-    auto wmin_of = [&](int64_t g) {
-      for (int j = 0; j < keys.n; ++j)
-        if (keys.k[j] == g) {
-          double v;
-          std::memcpy(&v, &m[j], sizeof(v));
-          return v;
-        }
-      return (double)INFINITY;  // not a group the quantiles fall in
-    };
-    grouped_quantiles(gc, value, wmin_of, P, 9, o + 19);
+    if (cubic) radii_quantiles(radii[b], c->dx, o + 19);
+    else
+      for (int i = 0; i < RADII_QUANTILES; ++i) o[19 + i] = NAN;
   }
-  return s;
+  return WDM_OK;
 }
 
 wdm_status wdm_interpolate_phi(wdm_ctx* c, const double* pos, int64_t n, double* out) {
