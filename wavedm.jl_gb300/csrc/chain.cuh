@@ -1,0 +1,32 @@
+// Kernels of one stream whose launches overlap.
+//
+// The passes of a step follow one another on a stream, and a small grid's pass
+// takes about as long as its launch.  They are launched with programmatic stream
+// serialisation: a pass's CTAs start, load the twiddle tables (which nothing writes
+// after a context's creation) and set up their barriers before the pass in front has
+// been retired, then wait here for its completion and its memory.  Every CTA
+// waits, so that a pass's completion implies the completion of all before it.  Nothing that another kernel or a copy writes is read before
+// the wait, and none of it through the non-coherent path (no __restrict__ on
+// pointers to it; it measured the same).
+//
+// When the next pass may start:
+// - As a rule once every CTA of this one has exited (no trigger).  A trigger at the
+//   start would let the next CTAs in beside the running ones, and they pile up on the
+//   SMs that have room instead of spreading: 384^3 1277 -> 1384 us a step, 256^3
+//   373 -> 422 (without overlap at all 1302 and 391).
+// - At the start in grids of at most CHAIN_SMALL threads, which leave most SMs empty
+//   in any case: 64^3 23.3 -> 21.1 us a step (without overlap 31.9), 48^3 23.3 -> 20.7.
+#pragma once
+
+namespace wdm {
+
+constexpr unsigned CHAIN_SMALL = 32768;
+
+template <bool TRIGGER>
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  if (TRIGGER && gridDim.x * gridDim.y * blockDim.x <= CHAIN_SMALL)
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+}  // namespace wdm

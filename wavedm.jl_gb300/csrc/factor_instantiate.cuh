@@ -24,9 +24,7 @@ struct Launch {
     const int tx = ge.edge ? ge.nxa / LINES : (ge.nxa + LINES - 1) / LINES;
     const long long tiles = ((long long)ge.rows * tx + ge.edge) * batch;
     const long long cap = (long long)resident_ctas<K>(NT, SMEM) * sm_count();
-    K<<<(unsigned)(tiles < cap ? tiles : cap), NT, SMEM, st>>>(data, map, emap, ge, tw, op, batch);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<K>(dim3((unsigned)(tiles < cap ? tiles : cap)), NT, SMEM, st, data, map, emap, ge, tw, op, batch);
   }
 
   // The line pass as the context's tuner chose it: the TMA pass where the
@@ -55,9 +53,7 @@ struct Launch {
     constexpr auto K = k_line_tile<N, MODE, Op>;
     cudaError_t e;
     if ((e = prep_once<K>(SMEM)) != cudaSuccess) return e;
-    K<<<dim3((g.nlines + LINES - 1) / LINES, batch), NT, SMEM, st>>>(data, g, tw, op);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<K>(dim3((g.nlines + LINES - 1) / LINES, batch), NT, SMEM, st, data, g, tw, op);
   }
   static cudaError_t line(float2* data, const LineGeom& g, const float4* tw, bool inv, int batch, cudaStream_t st) {
     return inv ? lines<1>(data, g, tw, None{}, batch, st) : lines<0>(data, g, tw, None{}, batch, st);
@@ -88,9 +84,7 @@ struct Launch {
     const long long per_sm = (units + sms - 1) / sms;
     const int warps = (int)(per_sm < R::WARPS ? per_sm : R::WARPS);
     const long long ctas = (units + warps - 1) / warps, cap = (long long)(R::KICK > R::RHO ? R::KICK : R::RHO) * sms;
-    K<<<(unsigned)(ctas < cap ? ctas : cap), 32 * warps, R::smem(warps), st>>>(args..., w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<K>(dim3((unsigned)(ctas < cap ? ctas : cap)), 32 * warps, R::smem(warps), st, args..., w);
   }
   static cudaError_t fft(float2* data, const RowGeom& rg, const float4* tw, bool inv, float scale, int batch,
                          cudaStream_t st) {
@@ -131,9 +125,7 @@ struct Launch {
     const int planes = p.rg.nrows / p.rg.ny * batch;
     const int fit = (int)(228 * 1024 / (smem + 1024));
     const int warps = planes <= sm_count() || fit <= 1 ? PLANE_WARPS : fit < 8 ? (PLANE_WARPS + fit - 1) / fit : 2;
-    K<<<planes, 32 * warps, smem, st>>>(p, a);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<K>(dim3(planes), 32 * warps, smem, st, p, a);
   }
   static cudaError_t plane_kick(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg,
                                 long long hpitch, long long hbstride, const float4* twx, const float4* twy,

@@ -1,6 +1,7 @@
 // Line passes (y and z axis) on the two-factor transforms of fft_factor.cuh: a
 // TMA-fed persistent kernel, and one register tile per CTA.
 #pragma once
+#include "chain.cuh"
 #include "fft_factor.cuh"
 #include "passes.cuh"
 
@@ -202,11 +203,12 @@ __device__ __forceinline__ void line_tile(float2* __restrict__ data, const LineG
 // the array has no tensor-map view, or the autotuner prefers it.
 template <int N, int MODE, class Op>
 __global__ void __launch_bounds__(line_threads<N>(), line_ctas<N>())
-k_line_tile(float2* __restrict__ data, LineGeom g, const float4* __restrict__ twg, Op op) {
+k_line_tile(float2* data, LineGeom g, const float4* __restrict__ twg, Op op) {
   extern __shared__ float2 smem[];
   float4* tw = reinterpret_cast<float4*>(smem);
   load_twiddles(tw, twg, N);
   if (MODE == 1) __syncthreads();  // else visible after the tile's first barrier
+  chain_wait<true>();
   line_tile<N, MODE, Op>(data, g, tw, op, blockIdx.x * LINES, blockIdx.y, smem + 2 * N, threadIdx.x);
 }
 
@@ -273,7 +275,7 @@ __device__ __forceinline__ void line_tma_prefetch(const CUtensorMap* map, const 
 
 template <int N, int MODE, class Op, bool LATE>
 __global__ void __launch_bounds__(line_threads<N>(), (line_tma_ctas_of<N>(line_tma_slots<N>(), sizeof(float))))
-k_line_tma(float2* __restrict__ data, const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap emap,
+k_line_tma(float2* data, const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap emap,
            LineGeom g, const float4* __restrict__ twg, Op op, int batch) {
   using TT = TmaTile<N>;
   constexpr int SLOTS = line_tma_slots<N>();
@@ -303,6 +305,7 @@ k_line_tma(float2* __restrict__ data, const __grid_constant__ CUtensorMap map, c
     mbar_fence_init();
   }
   load_twiddles(tw, twg, N);
+  chain_wait<false>();
   if constexpr (STAGED)
     for (int i = tid; i < N; i += blockDim.x) optab[i] = op.entry(i);
   __syncthreads();

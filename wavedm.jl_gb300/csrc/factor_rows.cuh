@@ -21,6 +21,7 @@
 // Bound by the FMA pipe, shared memory and DRAM at about half of each (the
 // Stockham row passes: by shared-memory wavefronts, 70-78% of the data pipe).
 #pragma once
+#include "chain.cuh"
 #include "fft_factor.cuh"
 #include "xpass_warp.cuh"
 
@@ -82,6 +83,7 @@ struct Warp {
     float4* t = reinterpret_cast<float4*>(smem);
     load_twiddles(t, twg, N);
     __syncthreads();
+    chain_wait<false>();
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
     set(t, smem + 2 * N + (size_t)warp * R::WORDS, w, blockIdx.x * warps + warp, gridDim.x * warps);
   }
@@ -190,7 +192,7 @@ __device__ __forceinline__ void split_half(const float2* va, const float2* vb, i
 
 // The pairs' packed lines from their half spectra, through stage B into E(0).
 template <int N>
-__device__ __forceinline__ void packed_in(const Warp<N>& w, const float2* __restrict__ H, long long hpitch,
+__device__ __forceinline__ void packed_in(const Warp<N>& w, const float2* H, long long hpitch,
                                           long long hbstride) {
   using R = Rows<N>;
   b_items<N, R::PW>(w, [&](int j, int k1) {
@@ -205,7 +207,7 @@ __device__ __forceinline__ void packed_in(const Warp<N>& w, const float2* __rest
 
 // The half spectra of the pairs' rows from their packed lines in E(0).
 template <int N>
-__device__ __forceinline__ void packed_out(const Warp<N>& w, float2* __restrict__ H, long long hpitch,
+__device__ __forceinline__ void packed_out(const Warp<N>& w, float2* H, long long hpitch,
                                            long long hbstride) {
   using R = Rows<N>;
   constexpr int RA = R::RA, RB = R::RB, ITEMS = R::PW * RA / 2;
@@ -341,7 +343,7 @@ __device__ __forceinline__ void kick_lane(At at, float2* x, const float2* psi_in
 }
 
 template <int N, bool FWD>
-__device__ __forceinline__ void kick_units(Warp<N>& w, const float2* psi_in, float2* psi, const float2* __restrict__ H,
+__device__ __forceinline__ void kick_units(Warp<N>& w, const float2* psi_in, float2* psi, const float2* H,
                                            const RowGeom& rg, long long hpitch, long long hbstride, const KickArgs& a) {
   using R = Rows<N>;
   constexpr int RA = R::RA, RB = R::RB;
@@ -374,7 +376,7 @@ __device__ __forceinline__ void kick_units(Warp<N>& w, const float2* psi_in, flo
 
 template <int N, bool FWD>
 __global__ void __launch_bounds__(32 * Rows<N>::WARPS, Rows<N>::KICK)
-k_rows_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, RowGeom rg, long long hpitch,
+k_rows_kick(const float2* psi_in, float2* psi, const float2* H, RowGeom rg, long long hpitch,
             long long hbstride, const float4* __restrict__ twg, KickArgs a, XWork work) {
   extern __shared__ __align__(16) float2 smem[];
   Warp<N> w(smem, twg, work);
@@ -385,7 +387,7 @@ k_rows_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, Row
 // density: psi x-inverse (+ mask), rho = |psi|^2 (+ rho_b) - shift, packed R2C -> H
 // ----------------------------------------------------------------------------
 // The pair is done: reduce its RB lanes' CentreAcc and add it to the pair's
-// CentreSum (on its first lane), as centre_pair_done does for a lane group.
+// CentreSum (on its first lane).
 template <int N>
 __device__ __forceinline__ void rows_centre_done(const RhoArgs& a, const RowGeom& rg, const CentreAcc& ca,
                                                  CentreSum& cs, int b, int ra, bool ok, int n2) {
@@ -523,7 +525,7 @@ __device__ __forceinline__ void rho_units(Warp<N>& w, float2* __restrict__ psi, 
 // CEN: also accumulate the density maximum and moments for the tide's frame
 template <int N, bool CEN>
 __global__ void __launch_bounds__(32 * Rows<N>::WARPS, Rows<N>::RHO)
-k_rows_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
+k_rows_rho(float2* psi, float2* H, RowGeom rg, long long hpitch, long long hbstride,
            const float4* __restrict__ twg, RhoArgs a, XWork work) {
   extern __shared__ __align__(16) float2 smem[];
   Warp<N> w(smem, twg, work);
@@ -536,7 +538,7 @@ k_rows_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long lo
 // C2C of every row, in place, scaled.
 template <int N, bool INV>
 __global__ void __launch_bounds__(32 * Rows<N>::WARPS, Rows<N>::RHO)
-k_rows_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg, float scale, XWork work) {
+k_rows_fft(float2* data, RowGeom rg, const float4* __restrict__ twg, float scale, XWork work) {
   using R = Rows<N>;
   constexpr int RA = R::RA, RB = R::RB;
   extern __shared__ __align__(16) float2 smem[];
@@ -571,7 +573,7 @@ k_rows_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg
 // Phi rows (real) from H.
 template <int N>
 __global__ void __launch_bounds__(32 * Rows<N>::WARPS, Rows<N>::RHO)
-k_rows_c2r(const float2* __restrict__ H, float* __restrict__ out, RowGeom rg, long long hpitch, long long hbstride,
+k_rows_c2r(const float2* H, float* out, RowGeom rg, long long hpitch, long long hbstride,
            const float4* __restrict__ twg, XWork work) {
   using R = Rows<N>;
   constexpr int RA = R::RA, RB = R::RB;
@@ -600,8 +602,8 @@ k_rows_c2r(const float2* __restrict__ H, float* __restrict__ out, RowGeom rg, lo
 // Real rows, minus a per-item shift, to half spectra.
 template <int N>
 __global__ void __launch_bounds__(32 * Rows<N>::WARPS, Rows<N>::RHO)
-k_rows_r2c(const float* __restrict__ in, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
-           const float4* __restrict__ twg, const float* __restrict__ shift_b, XWork work) {
+k_rows_r2c(const float* in, float2* H, RowGeom rg, long long hpitch, long long hbstride,
+           const float4* __restrict__ twg, const float* shift_b, XWork work) {
   using R = Rows<N>;
   constexpr int RA = R::RA, RB = R::RB;
   extern __shared__ __align__(16) float2 smem[];

@@ -33,6 +33,25 @@ static cudaError_t prep_once(size_t smem) {
   return v == 1 ? cudaSuccess : (cudaError_t)(v - 2);
 }
 
+// Launch K so that its CTAs may start while the stream's previous kernel drains
+// (chain.cuh: the kernel waits for that one itself).
+template <auto K, class... Args>
+static cudaError_t launch_chained(dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, K, args...);
+  ++tl_kernel_launches;
+  return cudaGetLastError();
+}
+
 // SMs of the current device.
 static int sm_count() {
   static std::atomic<int> n[MAX_DEVICES];
