@@ -32,9 +32,6 @@ enum {
   RED_SWR2,
   RED_FIELDS
 };
-// fields combined by max rather than by sum (RED_ARG travels with RED_MAX)
-__host__ __device__ constexpr bool red_is_max(int q) { return q == RED_MAX || q == RED_ARG || q == RED_PHIMAX; }
-
 struct RedGeom {
   int nx, ny, nz;
   double dx, dy, dz, x0, y0, z0;

@@ -32,7 +32,6 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-__device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 // multiply by -i (forward sign) or +i (inverse sign)
 template <bool INV>
@@ -383,20 +382,6 @@ template <int N, int T, int LP, bool INV, int... Rs>
 __device__ __forceinline__ void run_stages(Radices<Rs...>, float2* v, float2* s, const float4* tw, int t, int l) {
   run_stages_impl<N, T, LP, INV, (1 << 30), 1, 0, Rs...>(v, s, tw, t, l);
 }
-
-// Same with only line slots l < LACT exchanging through s.
-template <int N, int T, int LP, bool INV, int LACT, int... Rs>
-__device__ __forceinline__ void run_stages_act(Radices<Rs...>, float2* v, float2* s, const float4* tw, int t, int l) {
-  run_stages_impl<N, T, LP, INV, LACT, 1, 0, Rs...>(v, s, tw, t, l);
-}
-
-// cp.async: 8-byte global -> shared copies that do not pass through registers
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Position along the line of register slot (i, k) before the first stage of
 // radix R (the load pattern) or after the last stage of radix R (the store

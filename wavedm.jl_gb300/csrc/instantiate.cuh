@@ -24,52 +24,31 @@ struct Launch {
     return cudaGetLastError();
   }
 
-  // persistent line pass: one wave of resident CTAs walking all tiles
+  // the line pass as the tuner chose it
   template <int MODE, class Op>
-  static cudaError_t lpipe(float2* data, const LineGeom& g, const float4* tw, const Op& op, int batch,
+  static cudaError_t lines(float2* data, const LineGeom& g, const float4* tw, const Op& op, int batch,
                            cudaStream_t st) {
     if (g.nlines <= 0 || batch <= 0) return cudaSuccess;
-#if !defined(WDM_LINE_PIPELINE) && !defined(WDM_LINE_TILE)
-    {
-      CUtensorMap map, emap;
-      if (g.impl == LINE_IMPL_TMA && LineMaps<N>::line_map(&map, data, g, batch)) {
-        LineGeom ge = g;
-        ge.edge = 0;
-#ifndef WDM_NO_EDGE_TILES
-        if (LineMaps<N>::edge_map(&emap, data, g, batch)) ge.edge = g.rows / 8;
-#endif
-        if (!ge.edge) emap = map;  // not read
-        // The next tile's copy goes out late (k_lfft_tma) in the fused z
-        // passes, which are bound by instruction issue, and in the y passes
-        // of a half spectrum (the ones with edge tiles); early in the y passes
-        // of psi, which are bound by memory.  Measured at 384^3 against early
-        // everywhere: the z passes 0.8-1.1% faster, the half-spectrum y
-        // passes 1.3-3% faster; late everywhere made the psi y passes 0.7-1.3%
-        // slower.
-        if constexpr (MODE == 2) {
-          return ltma_launch<MODE, true>(data, map, emap, ge, tw, op, batch, st);
-        } else {
-#ifndef WDM_TMA_EARLY_HALF_Y  // tuning variant: early in every y pass
-          if (ge.edge) return ltma_launch<MODE, true>(data, map, emap, ge, tw, op, batch, st);
-#endif
-          return ltma_launch<MODE, false>(data, map, emap, ge, tw, op, batch, st);
-        }
+    CUtensorMap map, emap;
+    if (g.impl == LINE_IMPL_TMA && LineMaps<N>::line_map(&map, data, g, batch)) {
+      LineGeom ge = g;
+      ge.edge = LineMaps<N>::edge_map(&emap, data, g, batch) ? g.rows / 8 : 0;
+      if (!ge.edge) emap = map;  // not read
+      // The next tile's copy goes out late (k_lfft_tma) in the fused z
+      // passes, which are bound by instruction issue, and in the y passes
+      // of a half spectrum (the ones with edge tiles); early in the y passes
+      // of psi, which are bound by memory.  Measured at 384^3 against early
+      // everywhere: the z passes 0.8-1.1% faster, the half-spectrum y
+      // passes 1.3-3% faster; late everywhere made the psi y passes 0.7-1.3%
+      // slower.
+      if constexpr (MODE == 2) {
+        return ltma_launch<MODE, true>(data, map, emap, ge, tw, op, batch, st);
+      } else {
+        if (ge.edge) return ltma_launch<MODE, true>(data, map, emap, ge, tw, op, batch, st);
+        return ltma_launch<MODE, false>(data, map, emap, ge, tw, op, batch, st);
       }
     }
-#endif
-#ifndef WDM_LINE_PIPELINE
     return ltile<MODE>(data, g, tw, op, batch, st);
-#else
-    constexpr size_t SMEM = lpipe_smem_bytes<N, MODE>();
-    cudaError_t e;
-    if ((e = prep_once<k_lfft_pipe<N, MODE, Op>>(SMEM)) != cudaSuccess) return e;
-    const long long tiles = (long long)((g.nlines + LINES - 1) / LINES) * batch;
-    const long long cap = (long long)resident_ctas<k_lfft_pipe<N, MODE, Op>>(NT, SMEM) * sm_count();
-    const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-    k_lfft_pipe<N, MODE, Op><<<grid, NT, SMEM, st>>>(data, g, tw, op, batch);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
-#endif
   }
 
   // one register tile of LINES lines per CTA (lines may straddle rows)
@@ -85,15 +64,15 @@ struct Launch {
   }
 
   static cudaError_t lfft(float2* data, const LineGeom& g, const float4* tw, bool inv, int batch, cudaStream_t st) {
-    return inv ? lpipe<1>(data, g, tw, NoOp{}, batch, st) : lpipe<0>(data, g, tw, NoOp{}, batch, st);
+    return inv ? lines<1>(data, g, tw, NoOp{}, batch, st) : lines<0>(data, g, tw, NoOp{}, batch, st);
   }
   static cudaError_t lfft_drift(float2* data, const LineGeom& g, const float4* tw, const DriftOp& op, int batch,
                                 cudaStream_t st) {
-    return lpipe<2>(data, g, tw, op, batch, st);
+    return lines<2>(data, g, tw, op, batch, st);
   }
   static cudaError_t lfft_poisson(float2* data, const LineGeom& g, const float4* tw, const PoissonOp& op, int batch,
                                   cudaStream_t st) {
-    return lpipe<2>(data, g, tw, op, batch, st);
+    return lines<2>(data, g, tw, op, batch, st);
   }
   // x passes: lane group per row pair, grid-stride over warp units
   static constexpr int XNT = XCfg<N>::NT;
@@ -107,20 +86,14 @@ struct Launch {
     const long long cap = 152LL * 6;
     return dim3((unsigned)(ctas < cap ? ctas : cap));
   }
-  static cudaError_t xfft(float2* data, const RowGeom& rg, const float4* tw, bool inv, float scale, int batch,
-                          cudaStream_t st) {
+  // forward
+  static cudaError_t xfft(float2* data, const RowGeom& rg, const float4* tw, float scale, int batch, cudaStream_t st) {
     cudaError_t e;
     XWork w;
     const dim3 gr = grid_x(rg, batch, &w);
-    if (inv) {
-      if ((e = prep_once<k_xw_fft<N, true>>(XSMEM)) != cudaSuccess) return e;
-      k_xw_fft<N, true><<<gr, XNT, XSMEM, st>>>(data, rg, tw, scale, w);
-      ++tl_kernel_launches;
-    } else {
-      if ((e = prep_once<k_xw_fft<N, false>>(XSMEM)) != cudaSuccess) return e;
-      k_xw_fft<N, false><<<gr, XNT, XSMEM, st>>>(data, rg, tw, scale, w);
-      ++tl_kernel_launches;
-    }
+    if ((e = prep_once<k_xw_fft<N>>(XSMEM)) != cudaSuccess) return e;
+    k_xw_fft<N><<<gr, XNT, XSMEM, st>>>(data, rg, tw, scale, w);
+    ++tl_kernel_launches;
     return cudaGetLastError();
   }
   // Staged x passes: the layout conditions of their bulk copies.  Rows of
@@ -144,13 +117,12 @@ struct Launch {
     const long long cap = (long long)resident_ctas<K>(XNT, smem) * sm_count();
     return dim3((unsigned)(ctas < cap ? ctas : cap));
   }
-  template <bool CEN>
-  static cudaError_t x_inv_rho_t(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
-                                 const float4* tw, const RhoArgs& a, int batch, cudaStream_t st) {
+  static cudaError_t x_inv_rho(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
+                               const float4* tw, const RhoArgs& a, int batch, cudaStream_t st) {
     cudaError_t e;
     XWork w;
     if (x_staged_ok(rg, hpitch, psi, H, a.rho_b) && (!a.rho_b || (a.rb_bstride * 4) % 16 == 0)) {
-      constexpr auto K = k_xs_inv_rho<N, CEN>;
+      constexpr auto K = k_xs_inv_rho<N>;
       if ((e = prep_once<K>(XS::SMEM)) != cudaSuccess) return e;
       const dim3 gr = grid_xs<K>(rg, batch, &w);
       K<<<gr, XNT, XS::SMEM, st>>>(psi, H, rg, hpitch, hbstride, tw, a, w);
@@ -158,15 +130,10 @@ struct Launch {
       return cudaGetLastError();
     }
     const dim3 gr = grid_x(rg, batch, &w);
-    if ((e = prep_once<k_xw_inv_rho<N, CEN>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_inv_rho<N, CEN><<<gr, XNT, XSMEM, st>>>(psi, H, rg, hpitch, hbstride, tw, a, w);
+    if ((e = prep_once<k_xw_inv_rho<N>>(XSMEM)) != cudaSuccess) return e;
+    k_xw_inv_rho<N><<<gr, XNT, XSMEM, st>>>(psi, H, rg, hpitch, hbstride, tw, a, w);
     ++tl_kernel_launches;
     return cudaGetLastError();
-  }
-  static cudaError_t x_inv_rho(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
-                               const float4* tw, const RhoArgs& a, int batch, cudaStream_t st) {
-    return a.centre ? x_inv_rho_t<true>(psi, H, rg, hpitch, hbstride, tw, a, batch, st)
-                    : x_inv_rho_t<false>(psi, H, rg, hpitch, hbstride, tw, a, batch, st);
   }
   template <bool FWD>
   static cudaError_t x_kick_t(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg, long long hpitch,

@@ -19,9 +19,8 @@ struct KernelSet {
                             cudaStream_t st);
   cudaError_t (*lfft_poisson)(float2* data, const LineGeom& g, const float4* tw, const PoissonOp& op, int batch,
                               cudaStream_t st);
-  // contiguous rows (x axis)
-  cudaError_t (*xfft)(float2* data, const RowGeom& rg, const float4* tw, bool inv, float scale, int batch,
-                      cudaStream_t st);
+  // contiguous rows (x axis); xfft: forward
+  cudaError_t (*xfft)(float2* data, const RowGeom& rg, const float4* tw, float scale, int batch, cudaStream_t st);
   cudaError_t (*x_inv_rho)(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
                            const float4* tw, const RhoArgs& a, int batch, cudaStream_t st);
   cudaError_t (*x_kick)(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg, long long hpitch,

@@ -5,9 +5,7 @@
 //   H    complex64 [nz][ny][hpitch]    the density / potential half spectrum
 //                                      along x (nx/2 + 1 columns, Hermitian in
 //                                      kx; hpitch: that rounded up to even)
-// One KDK step is eight launches, each one read + one write of its array (the
-// line passes are k_lfft_tma, or k_lfft_tile; the x passes the staged k_xs_*
-// kernels of xpass_staged.cuh, or the direct k_xw_* kernels of xpass_warp.cuh):
+// One KDK step is eight passes, each one read + one write of its array:
 //   P1 kick       H -> Phi rows (C2R), psi <- exp(-i dt Phi) psi, x-FFT fwd
 //   P2 line <0>   psi, y axis
 //   P3 line <2>   psi, z axis: fwd, exp(-i k^2 dt/2)/(nx ny nz) (DriftOp), inverse
@@ -17,6 +15,12 @@
 //   P6 line <0>   H, y axis
 //   P7 line <2>   H, z axis: fwd, -c/(k^2 nx ny nz) (PoissonOp), inverse
 //   P8 line <1>   H, y axis
+// The step runs them on two-factor transforms (factor_lines.cuh, factor_rows.cuh),
+// or P8+P1+P2 and P4+P5+P6 as one launch each where a plane fits a CTA
+// (factor_planes.cuh).  Here and in xpass_warp.cuh and xpass_staged.cuh: the
+// arguments that both share, and the passes on Stockham transforms that the
+// adjoint keeps, because the gradient of a loss magnifies rounding: another order
+// of additions moves it by 1e-6 to 3e-4 of its value.
 #pragma once
 #include "fft_engine.cuh"
 #include "tma.cuh"
@@ -38,13 +42,6 @@ __host__ __device__ constexpr int min_blocks() {
   return threads_for<N>() >= 512 ? 1 : 512 / threads_for<N>();
 #endif
 }
-
-template <int N>
-__host__ __device__ constexpr size_t smem_bytes() { return sizeof(float2) * (size_t)(2 * N + N * LPITCH); }
-
-// fused forward/op/inverse line pass: both twiddle tables
-template <int N>
-__host__ __device__ constexpr size_t smem_bytes_mid() { return sizeof(float2) * (size_t)(4 * N + N * LPITCH); }
 
 struct LineGeom {
   int nlines;         // lines per batch item
@@ -93,12 +90,6 @@ __device__ __forceinline__ long long line_base(const LineGeom& g, int line) {
 // k-space operators applied between the forward and inverse transforms of a
 // fused pass at mode (mx, my, pos = mz) of batch item b.
 // ----------------------------------------------------------------------------
-// Exact error of the FP32 sum s = a + b (Knuth two-sum).
-__device__ __forceinline__ float two_sum_err(float a, float b, float s) {
-  const float bb = s - a;
-  return (a - (s - bb)) + (b - bb);
-}
-
 struct DriftOp {
   // precise form: the factor exp(-i (kx^2 + ky^2 + kz^2) dt/2) / (nx ny nz)
   // separates into a factor per z line and one per mode along the line.
@@ -236,103 +227,6 @@ __device__ __forceinline__ void lines_store(const float2* v, float2* base, long 
   for (int i = 0; i < N / (R * T); ++i)
 #pragma unroll
     for (int k = 0; k < R; ++k) base[(long long)slot_pos<N, T, R>(t, i, k) * ps] = v[i * R + k];
-}
-
-// Persistent, double-buffered line pass.  Each CTA walks tiles of LINES lines
-// (grid-stride over all batch items).  While tile i is transformed in
-// registers (its exchanges reuse the buffer it arrived in), the cp.async copy
-// of tile i+1 into the other buffer is in flight, so the loads of a CTA never
-// wait behind its own arithmetic.  Thread (t, l) copies exactly the points
-// t + T m of line l that its first stage reads; 16 lanes of a half-warp copy
-// 16 neighbouring lines at one point, i.e. 128 contiguous bytes when the lines
-// are contiguous along x.
-// MODE: 0 forward, 1 inverse, 2 forward / op / inverse (fused k-space step).
-constexpr int LBUF = LINES;  // pitch of a tile buffer: point-major, one slot per line
-
-template <int N, int MODE>
-__host__ __device__ constexpr size_t lpipe_smem_bytes() {
-  return sizeof(float4) * (MODE == 2 ? 2 : 1) * N + 2 * sizeof(float2) * (size_t)N * LBUF;
-}
-
-template <int N>
-__device__ __forceinline__ void lines_issue(float2* buf, const LineGeom& g, float2* data, long long tile,
-                                            int tiles_per_item, int t, int l) {
-  constexpr int T = Plan<N>::T;
-  const int b = (int)(tile / tiles_per_item);
-  const int line = (int)(tile - (long long)b * tiles_per_item) * LINES + l;
-  if (line >= g.nlines) return;
-  const float2* base = data + b * g.bstride + line_base(g, line);
-#pragma unroll
-  for (int m = 0; m < N / T; ++m) {
-    const int p = t + T * m;
-    cp_async8(buf + p * LBUF + l, base + (long long)p * g.pstride);
-  }
-}
-
-// The tiles base + sub, base + step + sub, ... (tile numbers over all batch
-// items) by the threads tid < threads_for<N>() of one group, with the group's
-// double buffer bufs (2 N LBUF entries) and the twiddle tables at tw: the
-// cp.async copy of the group's next tile is in flight while its current one is
-// transformed.  Every thread of the CTA runs the same rounds (a group without
-// a tile in a round computes on stale data and stores nothing), so the CTA's
-// barriers line up; the arithmetic is that of lfft_tile_one.
-template <int N, int MODE, class Op>
-__device__ __forceinline__ void lfft_pipe_run(float2* __restrict__ data, const LineGeom& g, const float4* tw,
-                                              const Op& op, int batch, float2* bufs, int tid, long long base,
-                                              long long step, int sub) {
-  using P = Plan<N>;
-  constexpr int T = P::T;
-  using Rad = typename P::Fwd;
-  using Rev = typename Reverse<Rad>::type;
-  constexpr int R1 = RadInfo<Rad>::first, RS = RadInfo<Rad>::last;
-  const int l = tid % LINES, t = tid / LINES;
-  const int tiles_per_item = (g.nlines + LINES - 1) / LINES;
-  const long long total = (long long)tiles_per_item * batch;
-  if (base + sub < total) lines_issue<N>(bufs, g, data, base + sub, tiles_per_item, t, l);
-  cp_async_commit();
-  int cur = 0;
-  for (; base < total; base += step) {
-    const long long tile = base + sub, nxt = tile + step;
-    if (nxt < total) lines_issue<N>(bufs + (cur ^ 1) * N * LBUF, g, data, nxt, tiles_per_item, t, l);
-    cp_async_commit();
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    __syncthreads();
-    float2* s = bufs + cur * N * LBUF;
-    const bool have = tile < total;
-    const int b = have ? (int)(tile / tiles_per_item) : 0;
-    const int line = have ? (int)(tile - (long long)b * tiles_per_item) * LINES + l : g.nlines;
-    const bool ok = line < g.nlines;
-    float2 v[N / T];
-    stage_read<N, T, R1, LBUF>(s, v, t, l);
-    if constexpr (MODE == 1) {
-      run_stages<N, T, LBUF, true>(Rad{}, v, s, tw, t, l);
-    } else {
-      run_stages<N, T, LBUF, false>(Rad{}, v, s, tw, t, l);
-    }
-    float2* gbase = data + b * g.bstride + (ok ? line_base(g, line) : 0);
-    if constexpr (MODE == 2) {
-      const int lc = ok ? line : 0;
-      const int mx = g.x0 + lc % g.nxa, my = lc / g.nxa;
-      op_points<N, T, RS, false>(op, v, mx, my, t, b, nullptr);
-      run_stages<N, T, LBUF, true>(Rev{}, v, s, tw + N, t, l);
-      lines_store<N, RadInfo<Rev>::last>(v, gbase, g.pstride, ok, t);
-    } else {
-      lines_store<N, RS>(v, gbase, g.pstride, ok, t);
-    }
-    __syncthreads();  // the exchanges in s are done before s receives the round after next
-    cur ^= 1;
-  }
-  cp_async_wait_all();
-}
-
-template <int N, int MODE, class Op>
-__global__ void __launch_bounds__(threads_for<N>(), min_blocks<N>())
-k_lfft_pipe(float2* __restrict__ data, LineGeom g, const float4* __restrict__ twg, Op op, int batch) {
-  extern __shared__ float2 smem[];
-  float4* tw = reinterpret_cast<float4*>(smem);  // line fwd [| line rev] tables
-  constexpr int NTAB = MODE == 2 ? 2 : 1;
-  load_twiddles(tw, twg + TW_LINE_FWD * N, NTAB * N);  // visible after the first round's barrier
-  lfft_pipe_run<N, MODE, Op>(data, g, tw, op, batch, smem + 2 * NTAB * N, threadIdx.x, blockIdx.x, gridDim.x, 0);
 }
 
 struct NoOp {
@@ -693,10 +587,6 @@ template <bool CONJ = false>
 __device__ __forceinline__ float2 kick_by(float2 v, float2 e, const KickArgs& a) {
   if (a.precise) return kick_by_t<true, CONJ>(v, e);
   return kick_by_t<false, CONJ>(v, e);
-}
-
-__device__ __forceinline__ float2 apply_kick(float2 v, float pot, const KickArgs& a) {
-  return kick_by(v, kick_factor(pot, a), a);
 }
 
 }  // namespace wdm

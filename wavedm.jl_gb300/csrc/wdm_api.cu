@@ -1908,7 +1908,7 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
   }
   cudaError_t e = launch_adj_seed(c->psi, c->rho_t, c->lam, c->ncell, B, c->dx * c->dy * c->dz, c->adj_acc, c->st);
   if (e != cudaSuccess) return cuda_fail(c, e, "adjoint seed");
-  if ((e = c->kx->xfft(c->lam, rows_psi(c), c->twx, false, (float)(1.0 / c->d.nx), B, c->st)) != cudaSuccess)
+  if ((e = c->kx->xfft(c->lam, rows_psi(c), c->twx, (float)(1.0 / c->d.nx), B, c->st)) != cudaSuccess)
     return cuda_fail(c, e, "adjoint x fwd");
   AdjArgs j{};
   j.D6 = tidal_dir ? c->D6 : nullptr;

@@ -241,8 +241,7 @@ k_xs_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, RowGe
 }
 
 // P5 (staged): psi x-inverse (+mask), rho = |psi|^2 (+rho_b) - shift, packed R2C -> H
-// (CEN: with the density maximum and moments for the tide's frame).
-template <int N, bool CEN>
+template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, XStage<N>::MINB)
 k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
              const float4* __restrict__ twg, RhoArgs a, XWork w) {
@@ -278,8 +277,6 @@ k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long 
     for (int r = 0; r < S::ROWS; ++r)
       if ((m >> r) & 1u) bulk_g2s(rbslot + r * S::RB_P, src + r * rg.pitch, (unsigned)(N * sizeof(float)), &xbar[0]);
   };
-  CentreSum cs;
-  cs.reset(-1);
   long long u = (long long)blockIdx.x * C::WARPS + warp;
   unsigned mcur = u < nunits ? rb_mask(u) : 0u;
   if (u < nunits) {
@@ -299,8 +296,6 @@ k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long 
     float rho0[N / T];  // row A density at radix-RS slots
     float2 z[N / T];    // packed (rho_A, rho_B) at radix-RS slots
     float2 v[N / T];
-    CentreAcc ca;
-    ca.reset();
     if (!WDM_XSTAGE_WAIT(1)) WDM_XSTAGE_FAIL(a.err);
     auto release_p = [&]() {
       xrelease();
@@ -336,8 +331,8 @@ k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long 
       release_p();
       if (with_rb && !WDM_XSTAGE_WAIT(0)) WDM_XSTAGE_FAIL(a.err);
       float2* rowa = psi + b * rg.bstride + (long long)ra * rg.pitch;
-      rho_row_post<N, CEN>(v, a, rg, ra, true, rowa, rb_of(0), shift, 0, rho0, z, t, ca);
-      rho_row_post<N, CEN>(vb, a, rg, ra + 1, true, rowa + rg.pitch, rb_of(1), shift, 1, rho0, z, t, ca);
+      rho_row_post<N>(v, a, rg, ra, true, rowa, rb_of(0), shift, 0, rho0, z, t);
+      rho_row_post<N>(vb, a, rg, ra + 1, true, rowa + rg.pitch, rb_of(1), shift, 1, rho0, z, t);
       if (with_rb) release_r();
     } else {
 #pragma unroll
@@ -357,19 +352,17 @@ k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long 
       if (half == 1) release_p();
       if (half == 0 && with_rb && !WDM_XSTAGE_WAIT(0)) WDM_XSTAGE_FAIL(a.err);
       const int r = ra + half;
-      inv_rho_row<N, CEN>(v, a, rg, r, true, psi + b * rg.bstride + (long long)r * rg.pitch, rb_of(half), shift,
-                          half, rho0, z, buf, tw, t, ca);
+      inv_rho_row<N>(v, a, rg, r, true, psi + b * rg.bstride + (long long)r * rg.pitch, rb_of(half), shift,
+                          half, rho0, z, buf, tw, t);
       if (half == 1 && with_rb) release_r();
     }
     }
-    if constexpr (CEN) centre_pair_done<N>(a, rg, ca, cs, b, ra, true, t);
     mcur = mnext;
     reorder<N, T, RS, R1>(z, v);
     run_wstages<N, T, C::NP, false>(Rad{}, v, buf, tw, t);
     float2* hrow = H + b * hbstride + ra * hpitch;
     store_packed_half<N, T, RS>(v, buf, hrow, hrow + hpitch, true, t);
   }
-  if (CEN && t == 0) cs.flush(a.centre);
 }
 
 // Adjoint kick (staged): the arithmetic of k_xw_adj_kick, with the H rows in

@@ -530,43 +530,6 @@ struct CentreSum {
   }
 };
 
-// The row pair (ra, ra + 1) of item b is done: reduce its lanes' CentreAcc over
-// the lane group (T lanes) and add it to the group's CentreSum (on lane t = 0).
-template <int N>
-__device__ __forceinline__ void centre_pair_done(const RhoArgs& a, const RowGeom& rg, const CentreAcc& ca,
-                                                 CentreSum& cs, int b, int ra, bool ok, int t) {
-  constexpr int T = XCfg<N>::T;
-  float best = ca.best, s0a = ca.s0[0], s0b = ca.s0[1], si = ca.si;
-  unsigned cell = ca.cell;
-#pragma unroll
-  for (int off = T / 2; off > 0; off >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, off, T);
-    const unsigned oc = __shfl_xor_sync(0xffffffffu, cell, off, T);
-    if (ob > best || (ob == best && oc < cell)) {
-      best = ob;
-      cell = oc;
-    }
-    s0a += __shfl_xor_sync(0xffffffffu, s0a, off, T);
-    s0b += __shfl_xor_sync(0xffffffffu, s0b, off, T);
-    si += __shfl_xor_sync(0xffffffffu, si, off, T);
-  }
-  if (t != 0 || !ok) return;
-  if (cs.item != b) {
-    cs.flush(a.centre);
-    cs.reset(b);
-  }
-  const int ja = ra % rg.ny, ka = ra / rg.ny, jb = (ra + 1) % rg.ny, kb = (ra + 1) / rg.ny;
-  cs.s0 += (double)s0a + (double)s0b;
-  cs.si += (double)si;
-  cs.sj += (double)s0a * ja + (double)s0b * jb;
-  cs.sk += (double)s0a * ka + (double)s0b * kb;
-  if (best >= 0.f) {
-    const unsigned long long key =
-        ((unsigned long long)__float_as_uint(best) << 32) | (unsigned long long)(0xffffffffu - cell);
-    if (key > cs.key) cs.key = key;
-  }
-}
-
 // The slice of an x pass one warp runs: warp units u0, u0 + ustride, ...,
 // with the twiddle tables of the pass (x fwd | x rev) in shared memory at tw
 // and this lane group's exchange buffer (XCfg<N>::NP entries) at buf.
@@ -638,10 +601,10 @@ k_xw_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, RowGe
 // space at radix-RS slots; mask it and store it back to `row` (write_psi), then
 // form rho - shift into rho0 (half 0) or the packed z (half 1).  rb: the
 // baryon density row or null.
-template <int N, bool CEN>
+template <int N>
 __device__ __forceinline__ void rho_row_post(float2* v, const RhoArgs& a, const RowGeom& rg, int r, bool ok,
                                              float2* row, const float* rb, float shift, int half, float* rho0,
-                                             float2* z, int t, CentreAcc& ca) {
+                                             float2* z, int t) {
   constexpr int T = XCfg<N>::T;
   constexpr int RS = RadInfo<typename XPlan<N>::Fwd>::last;
   if (a.write_psi) {
@@ -670,15 +633,6 @@ __device__ __forceinline__ void rho_row_post(float2* v, const RhoArgs& a, const 
     for (int q = 0; q < NQ; ++q) bad |= !isfinite(d(q));
     if (bad) *a.nonfinite = 1;
   }
-  if constexpr (CEN) {
-#pragma unroll
-    for (int i = 0; i < N / (RS * T); ++i)
-#pragma unroll
-      for (int k = 0; k < RS; ++k) {
-        const int x = slot_pos<N, T, RS>(t, i, k);
-        ca.add(d(i * RS + k), (unsigned)r * (unsigned)N + (unsigned)x, x, half);
-      }
-  }
   if (rb && ok) {
 #pragma unroll
     for (int i = 0; i < N / (RS * T); ++i)
@@ -692,16 +646,16 @@ __device__ __forceinline__ void rho_row_post(float2* v, const RhoArgs& a, const 
 // One row of P5: v holds psi row r (write_psi: x-spectral at radix-R1 slots,
 // else real space at radix-RS slots).  Inverts it (write_psi), then
 // rho_row_post.
-template <int N, bool CEN>
+template <int N>
 __device__ __forceinline__ void inv_rho_row(float2* v, const RhoArgs& a, const RowGeom& rg, int r, bool ok,
                                             float2* row, const float* rb, float shift, int half, float* rho0,
-                                            float2* z, float2* buf, const float4* tw, int t, CentreAcc& ca) {
+                                            float2* z, float2* buf, const float4* tw, int t) {
   using C = XCfg<N>;
   if (a.write_psi) run_wstages<N, C::T, C::NP, true>(typename XPlan<N>::Fwd{}, v, buf, tw, t);
-  rho_row_post<N, CEN>(v, a, rg, r, ok, row, rb, shift, half, rho0, z, t, ca);
+  rho_row_post<N>(v, a, rg, r, ok, row, rb, shift, half, rho0, z, t);
 }
 
-template <int N, bool CEN>
+template <int N>
 __device__ __forceinline__ void xw_inv_rho_units(float2* __restrict__ psi, float2* __restrict__ H, const RowGeom& rg,
                                                  long long hpitch, long long hbstride, const RhoArgs& a,
                                                  const XWork& w, const XSlice& sl) {
@@ -713,8 +667,6 @@ __device__ __forceinline__ void xw_inv_rho_units(float2* __restrict__ psi, float
   const float4* tw = sl.tw;
   float2* buf = sl.buf;
   const long long nunits = w.units(C::GROUPS);
-  CentreSum cs;
-  cs.reset(-1);
   for (long long u = sl.u0; u < nunits; u += sl.ustride) {
     const long long pp = u * C::GROUPS + g;
     const bool ok = pp < (long long)w.pairs_per_item * w.batch;
@@ -724,8 +676,6 @@ __device__ __forceinline__ void xw_inv_rho_units(float2* __restrict__ psi, float
     float rho0[N / T];  // row A density at radix-RS slots
     float2 z[N / T];    // packed (rho_A, rho_B) at radix-RS slots
     float2 v[N / T];
-    CentreAcc ca;
-    ca.reset();
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int r = ra + half;
@@ -743,33 +693,28 @@ __device__ __forceinline__ void xw_inv_rho_units(float2* __restrict__ psi, float
       }
       const bool rb_row = a.rho_b && (!a.rb_rows || a.rb_rows[r]);  // rows without baryon mass are zero
       const float* rb = rb_row ? a.rho_b + b * a.rb_bstride + (long long)r * rg.pitch : nullptr;
-      inv_rho_row<N, CEN>(v, a, rg, r, ok, row, rb, shift, half, rho0, z, buf, tw, t, ca);
+      inv_rho_row<N>(v, a, rg, r, ok, row, rb, shift, half, rho0, z, buf, tw, t);
     }
-    if constexpr (CEN) centre_pair_done<N>(a, rg, ca, cs, b, ra, ok, t);
     reorder<N, T, RS, R1>(z, v);
     run_wstages<N, T, C::NP, false>(Rad{}, v, buf, tw, t);
     float2* hrow = H + b * hbstride + ra * hpitch;
     store_packed_half<N, T, RS>(v, buf, hrow, hrow + hpitch, ok, t);
   }
-  if (CEN && t == 0) cs.flush(a.centre);
 }
 
-// CEN: also accumulate the density maximum and moments for the tide's frame
-// (RhoArgs::centre), a compile-time choice so that the pass without it keeps
-// its registers and instructions.
-template <int N, bool CEN>
+template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
 k_xw_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
              const float4* __restrict__ twg, RhoArgs a, XWork w) {
   WDM_XPASS_PROLOGUE
   (void)nunits;
   (void)t;
-  xw_inv_rho_units<N, CEN>(psi, H, rg, hpitch, hbstride, a, w,
+  xw_inv_rho_units<N>(psi, H, rg, hpitch, hbstride, a, w,
                            XSlice{(long long)blockIdx.x * C::WARPS + warp, wstride, tw, buf});
 }
 
-// Plain C2C x pass (rows processed pairwise, scaled output).
-template <int N, bool INV>
+// Plain forward C2C x pass (rows processed pairwise, scaled output).
+template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
 k_xw_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg, float scale, XWork w) {
   WDM_XPASS_PROLOGUE
@@ -786,7 +731,7 @@ k_xw_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg, 
       for (int i = 0; i < N / (R1 * T); ++i)
 #pragma unroll
         for (int k = 0; k < R1; ++k) v[i * R1 + k] = ok ? row[slot_pos<N, T, R1>(t, i, k)] : make_float2(0.f, 0.f);
-      run_wstages<N, T, C::NP, INV>(Rad{}, v, buf, tw, t);
+      run_wstages<N, T, C::NP, false>(Rad{}, v, buf, tw, t);
       if (ok)
 #pragma unroll
         for (int i = 0; i < N / (RS * T); ++i)
