@@ -16,6 +16,7 @@
 #include "ensemble.cuh"
 #include "factor_lines.cuh"
 #include "factor_rows.cuh"
+#include "launch_util.cuh"
 
 #include <algorithm>
 
@@ -236,8 +237,9 @@ size_t smem_for_axis(int n, int kind) {  // kind 0: x pass, else lines
   return 0;
 }
 
-__global__ void k_tide_frame(const unsigned long long* __restrict__ words, KickArgs a, int mode, int nx, int ny,
-                             int batch, float* __restrict__ frame) {
+__global__ void k_tide_frame(const unsigned long long* words, KickArgs a, int mode, int nx, int ny,
+                             int batch, float* frame) {
+  chain_wait<true>();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += gridDim.x * blockDim.x) {
     float T6[6];
     for (int q = 0; q < 6; ++q) T6[q] = a.T6b ? a.T6b[6 * b + q] : a.T6[q];
@@ -250,9 +252,7 @@ __global__ void k_tide_frame(const unsigned long long* __restrict__ words, KickA
 
 cudaError_t launch_tide_frame(const unsigned long long* words, const KickArgs& a, int mode, int nx, int ny, int batch,
                               float* frame, cudaStream_t st) {
-  k_tide_frame<<<(batch + 127) / 128, 128, 0, st>>>(words, a, mode, nx, ny, batch, frame);
-  ++tl_kernel_launches;
-  return cudaGetLastError();
+  return launch_chained<k_tide_frame>(dim3((batch + 127) / 128), 128, 0, st, words, a, mode, nx, ny, batch, frame);
 }
 
 bool ens_size_supported(int n) {

@@ -19,9 +19,7 @@ struct Launch {
     const long long tiles = ((long long)ge.rows * tx + ge.edge) * batch;
     const long long cap = (long long)resident_ctas<k_lfft_tma<N, MODE, Op, LATE>>(NT, SMEM) * sm_count();
     const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-    k_lfft_tma<N, MODE, Op, LATE><<<grid, NT, SMEM, st>>>(data, map, emap, ge, tw, op, batch);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_lfft_tma<N, MODE, Op, LATE>>(dim3(grid), NT, SMEM, st, data, map, emap, ge, tw, op, batch);
   }
 
   // the line pass as the tuner chose it
@@ -58,9 +56,7 @@ struct Launch {
     constexpr size_t SMEM = ltile_smem_bytes<N, MODE>();
     cudaError_t e;
     if ((e = prep_once<k_lfft_tile<N, MODE, Op>>(SMEM)) != cudaSuccess) return e;
-    k_lfft_tile<N, MODE, Op><<<dim3((g.nlines + LINES - 1) / LINES, batch), NT, SMEM, st>>>(data, g, tw, op);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_lfft_tile<N, MODE, Op>>(dim3((g.nlines + LINES - 1) / LINES, batch), NT, SMEM, st, data, g, tw, op);
   }
 
   static cudaError_t lfft(float2* data, const LineGeom& g, const float4* tw, bool inv, int batch, cudaStream_t st) {
@@ -92,9 +88,7 @@ struct Launch {
     XWork w;
     const dim3 gr = grid_x(rg, batch, &w);
     if ((e = prep_once<k_xw_fft<N>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_fft<N><<<gr, XNT, XSMEM, st>>>(data, rg, tw, scale, w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_xw_fft<N>>(gr, XNT, XSMEM, st, data, rg, tw, scale, w);
   }
   // Staged x passes: the layout conditions of their bulk copies.  Rows of
   // 16-byte multiples at 16-byte aligned addresses (the half spectrum with the
@@ -125,15 +119,11 @@ struct Launch {
       constexpr auto K = k_xs_inv_rho<N>;
       if ((e = prep_once<K>(XS::SMEM)) != cudaSuccess) return e;
       const dim3 gr = grid_xs<K>(rg, batch, &w);
-      K<<<gr, XNT, XS::SMEM, st>>>(psi, H, rg, hpitch, hbstride, tw, a, w);
-      ++tl_kernel_launches;
-      return cudaGetLastError();
+      return launch_chained<K>(gr, XNT, XS::SMEM, st, psi, H, rg, hpitch, hbstride, tw, a, w);
     }
     const dim3 gr = grid_x(rg, batch, &w);
     if ((e = prep_once<k_xw_inv_rho<N>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_inv_rho<N><<<gr, XNT, XSMEM, st>>>(psi, H, rg, hpitch, hbstride, tw, a, w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_xw_inv_rho<N>>(gr, XNT, XSMEM, st, psi, H, rg, hpitch, hbstride, tw, a, w);
   }
   template <bool FWD>
   static cudaError_t x_kick_t(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg, long long hpitch,
@@ -144,15 +134,11 @@ struct Launch {
       constexpr auto K = k_xs_kick<N, FWD>;
       if ((e = prep_once<K>(XS::SMEM)) != cudaSuccess) return e;
       const dim3 gr = grid_xs<K>(rg, batch, &w);
-      K<<<gr, XNT, XS::SMEM, st>>>(psi_in, psi, H, rg, hpitch, hbstride, tw, a, w);
-      ++tl_kernel_launches;
-      return cudaGetLastError();
+      return launch_chained<K>(gr, XNT, XS::SMEM, st, psi_in, psi, H, rg, hpitch, hbstride, tw, a, w);
     }
     const dim3 gr = grid_x(rg, batch, &w);
     if ((e = prep_once<k_xw_kick<N, FWD>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_kick<N, FWD><<<gr, XNT, XSMEM, st>>>(psi_in, psi, H, rg, hpitch, hbstride, tw, a, w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_xw_kick<N, FWD>>(gr, XNT, XSMEM, st, psi_in, psi, H, rg, hpitch, hbstride, tw, a, w);
   }
   static cudaError_t x_kick(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg, long long hpitch,
                             long long hbstride, const float4* tw, const KickArgs& a, bool fwd, int batch,
@@ -166,9 +152,7 @@ struct Launch {
     XWork w;
     const dim3 gr = grid_x(rg, batch, &w);
     if ((e = prep_once<k_xw_c2r<N>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_c2r<N><<<gr, XNT, XSMEM, st>>>(H, out, rg, hpitch, hbstride, tw, w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_xw_c2r<N>>(gr, XNT, XSMEM, st, H, out, rg, hpitch, hbstride, tw, w);
   }
   static cudaError_t x_r2c(const float* in, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
                            const float4* tw, const float* shift, int batch, cudaStream_t st) {
@@ -176,9 +160,7 @@ struct Launch {
     XWork w;
     const dim3 gr = grid_x(rg, batch, &w);
     if ((e = prep_once<k_xw_r2c<N>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_r2c<N><<<gr, XNT, XSMEM, st>>>(in, H, rg, hpitch, hbstride, tw, shift, w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_xw_r2c<N>>(gr, XNT, XSMEM, st, in, H, rg, hpitch, hbstride, tw, shift, w);
   }
   // host: the four stage-major twiddle tables of this axis length (TW_TABLES x N)
   static void fill_twiddles(float4* out) {
@@ -206,16 +188,12 @@ struct Launch {
         constexpr auto K = k_xs_adj_kick<N>;
         if ((e = prep_once<K>(XA::SMEM)) != cudaSuccess) return e;
         const dim3 gr = grid_xs<K>(rg, batch, &w, XA::SMEM);
-        K<<<gr, XNT, XA::SMEM, st>>>(lam, H, Hmu, rg, hpitch, hbstride, tw, a, j, w);
-        ++tl_kernel_launches;
-        return cudaGetLastError();
+        return launch_chained<K>(gr, XNT, XA::SMEM, st, lam, H, Hmu, rg, hpitch, hbstride, tw, a, j, w);
       }
     }
     const dim3 gr = grid_x(rg, batch, &w);
     if ((e = prep_once<k_xw_adj_kick<N>>(XSMEM)) != cudaSuccess) return e;
-    k_xw_adj_kick<N><<<gr, XNT, XSMEM, st>>>(lam, H, Hmu, rg, hpitch, hbstride, tw, a, j, w);
-    ++tl_kernel_launches;
-    return cudaGetLastError();
+    return launch_chained<k_xw_adj_kick<N>>(gr, XNT, XSMEM, st, lam, H, Hmu, rg, hpitch, hbstride, tw, a, j, w);
   }
   static cudaError_t adj_apply(float2* lam, const float2* Hmu, const RowGeom& rg, long long hpitch, long long hbstride,
                                const float4* tw, const AdjArgs& j, bool fwd, int batch, cudaStream_t st) {
@@ -224,14 +202,10 @@ struct Launch {
     const dim3 gr = grid_x(rg, batch, &w);
     if (fwd) {
       if ((e = prep_once<k_xw_adj_apply<N, true>>(XSMEM)) != cudaSuccess) return e;
-      k_xw_adj_apply<N, true><<<gr, XNT, XSMEM, st>>>(lam, Hmu, rg, hpitch, hbstride, tw, j, w);
-      ++tl_kernel_launches;
-    } else {
-      if ((e = prep_once<k_xw_adj_apply<N, false>>(XSMEM)) != cudaSuccess) return e;
-      k_xw_adj_apply<N, false><<<gr, XNT, XSMEM, st>>>(lam, Hmu, rg, hpitch, hbstride, tw, j, w);
-      ++tl_kernel_launches;
+      return launch_chained<k_xw_adj_apply<N, true>>(gr, XNT, XSMEM, st, lam, Hmu, rg, hpitch, hbstride, tw, j, w);
     }
-    return cudaGetLastError();
+    if ((e = prep_once<k_xw_adj_apply<N, false>>(XSMEM)) != cudaSuccess) return e;
+    return launch_chained<k_xw_adj_apply<N, false>>(gr, XNT, XSMEM, st, lam, Hmu, rg, hpitch, hbstride, tw, j, w);
   }
   static const KernelSet* set() {
     static const KernelSet ks = {N,          &lfft,  &lfft_drift,    &lfft_poisson, &xfft,     &x_inv_rho,

@@ -22,6 +22,7 @@
 // adjoint keeps, because the gradient of a loss magnifies rounding: another order
 // of additions moves it by 1e-6 to 3e-4 of its value.
 #pragma once
+#include "chain.cuh"
 #include "fft_engine.cuh"
 #include "tma.cuh"
 #include "wdm_math.cuh"
@@ -279,11 +280,12 @@ __device__ __forceinline__ void lfft_tile_one(float2* __restrict__ data, const L
 // tuning.
 template <int N, int MODE, class Op>
 __global__ void __launch_bounds__(threads_for<N>(), min_blocks<N>())
-k_lfft_tile(float2* __restrict__ data, LineGeom g, const float4* __restrict__ twg, Op op) {
+k_lfft_tile(float2* data, LineGeom g, const float4* twg, Op op) {
   constexpr int NTAB = MODE == 2 ? 2 : 1;
   extern __shared__ float2 smem[];
   float4* tw = reinterpret_cast<float4*>(smem);  // line fwd [| line rev] tables
   float2* s = smem + 2 * NTAB * N;
+  chain_wait<false>();
   load_twiddles(tw, twg + TW_LINE_FWD * N, NTAB * N);
   lfft_tile_one<N, MODE, Op>(data, g, tw, op, blockIdx.x * LINES, blockIdx.y, s, threadIdx.x);
 }
@@ -354,8 +356,8 @@ __host__ __device__ constexpr int ltma_min_blocks() {
 
 template <int N, int MODE, class Op, bool LATE>
 __global__ void __launch_bounds__(threads_for<N>(), ltma_min_blocks<N>())
-k_lfft_tma(float2* __restrict__ data, const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap emap,
-           LineGeom g, const float4* __restrict__ twg, Op op, int batch) {
+k_lfft_tma(float2* data, const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap emap,
+           LineGeom g, const float4* twg, Op op, int batch) {
   using P = Plan<N>;
   using TT = TmaTile<N>;
   constexpr int T = P::T;
@@ -387,6 +389,7 @@ k_lfft_tma(float2* __restrict__ data, const __grid_constant__ CUtensorMap map, c
     mbar_init(&bar[1], 1);
     mbar_fence_init();
   }
+  chain_wait<false>();
   load_twiddles(tw, twg + TW_LINE_FWD * N, NTAB * N);
   if constexpr (MODE == 2 && Op::TABLE)
     for (int i = tid; i < N; i += blockDim.x) optab[i] = op.table_entry(i);

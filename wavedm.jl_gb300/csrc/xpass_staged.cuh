@@ -143,8 +143,8 @@ __device__ __forceinline__ void unit_rows(long long u, int groups, int ppi, int*
 // P1 (staged): Phi rows from H, kick, forward x transform (FWD) or not.
 template <int N, bool FWD>
 __global__ void __launch_bounds__(XCfg<N>::NT, XStage<N>::MINB)
-k_xs_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, RowGeom rg, long long hpitch,
-          long long hbstride, const float4* __restrict__ twg, KickArgs a, XWork w) {
+k_xs_kick(const float2* psi_in, float2* psi, const float2* H, RowGeom rg, long long hpitch,
+          long long hbstride, const float4* twg, KickArgs a, XWork w) {
   WDM_XPASS_PROLOGUE
   WDM_XSTAGE_PROLOGUE
   auto issue_h = [&](long long u) {
@@ -243,8 +243,8 @@ k_xs_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, RowGe
 // P5 (staged): psi x-inverse (+mask), rho = |psi|^2 (+rho_b) - shift, packed R2C -> H
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, XStage<N>::MINB)
-k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
-             const float4* __restrict__ twg, RhoArgs a, XWork w) {
+k_xs_inv_rho(float2* psi, float2* H, RowGeom rg, long long hpitch, long long hbstride,
+             const float4* twg, RhoArgs a, XWork w) {
   WDM_XPASS_PROLOGUE
   WDM_XSTAGE_PROLOGUE
   float* rbslot = reinterpret_cast<float*>(slotA);
@@ -371,8 +371,8 @@ k_xs_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long 
 // straight to global memory.
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, XStageAdj<N>::MINB)
-k_xs_adj_kick(float2* __restrict__ lam, const float2* __restrict__ H, float2* __restrict__ Hmu, RowGeom rg,
-              long long hpitch, long long hbstride, const float4* __restrict__ twg, KickArgs a, AdjArgs j,
+k_xs_adj_kick(float2* lam, const float2* H, float2* Hmu, RowGeom rg,
+              long long hpitch, long long hbstride, const float4* twg, KickArgs a, AdjArgs j,
               XWork w) {
   WDM_XPASS_PROLOGUE
   WDM_XSTAGE_PROLOGUE_T(XStageAdj<N>)

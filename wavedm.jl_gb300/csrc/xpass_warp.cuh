@@ -375,6 +375,7 @@ __device__ __forceinline__ void store_packed_half(const float2* v, float2* buf, 
   (void)R1;                                                                         \
   (void)RS;                                                                         \
   extern __shared__ float2 smem[];                                                  \
+  chain_wait<false>();                                                              \
   WDM_XPASS_TWIDDLES                                                                \
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;                       \
   const int g = lane / T, t = lane % T;                                             \
@@ -583,8 +584,8 @@ __device__ __forceinline__ void xw_kick_units(const float2* psi_in, float2* psi,
 
 template <int N, bool FWD>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_kick(const float2* psi_in, float2* psi, const float2* __restrict__ H, RowGeom rg, long long hpitch,
-          long long hbstride, const float4* __restrict__ twg, KickArgs a, XWork w) {
+k_xw_kick(const float2* psi_in, float2* psi, const float2* H, RowGeom rg, long long hpitch,
+          long long hbstride, const float4* twg, KickArgs a, XWork w) {
   // psi_in == psi runs in place; a separate psi_in keeps the input state
   WDM_XPASS_PROLOGUE
   (void)nunits;
@@ -704,8 +705,8 @@ __device__ __forceinline__ void xw_inv_rho_units(float2* __restrict__ psi, float
 
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
-             const float4* __restrict__ twg, RhoArgs a, XWork w) {
+k_xw_inv_rho(float2* psi, float2* H, RowGeom rg, long long hpitch, long long hbstride,
+             const float4* twg, RhoArgs a, XWork w) {
   WDM_XPASS_PROLOGUE
   (void)nunits;
   (void)t;
@@ -716,7 +717,7 @@ k_xw_inv_rho(float2* __restrict__ psi, float2* __restrict__ H, RowGeom rg, long 
 // Plain forward C2C x pass (rows processed pairwise, scaled output).
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg, float scale, XWork w) {
+k_xw_fft(float2* data, RowGeom rg, const float4* twg, float scale, XWork w) {
   WDM_XPASS_PROLOGUE
   for (long long u = (long long)blockIdx.x * C::WARPS + warp; u < nunits; u += wstride) {
     const long long pp = u * C::GROUPS + g;
@@ -744,8 +745,8 @@ k_xw_fft(float2* __restrict__ data, RowGeom rg, const float4* __restrict__ twg, 
 // Phi rows (real) from H: packed C2R only.
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_c2r(const float2* __restrict__ H, float* __restrict__ out, RowGeom rg, long long hpitch, long long hbstride,
-         const float4* __restrict__ twg, XWork w) {
+k_xw_c2r(const float2* H, float* out, RowGeom rg, long long hpitch, long long hbstride,
+         const float4* twg, XWork w) {
   WDM_XPASS_PROLOGUE
   for (long long u = (long long)blockIdx.x * C::WARPS + warp; u < nunits; u += wstride) {
     const long long pp = u * C::GROUPS + g;
@@ -772,8 +773,8 @@ k_xw_c2r(const float2* __restrict__ H, float* __restrict__ out, RowGeom rg, long
 // Real rows -> H (packed R2C) from a float field, minus a per-item shift.
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_r2c(const float* __restrict__ in, float2* __restrict__ H, RowGeom rg, long long hpitch, long long hbstride,
-         const float4* __restrict__ twg, const float* __restrict__ shift_b, XWork w) {
+k_xw_r2c(const float* in, float2* H, RowGeom rg, long long hpitch, long long hbstride,
+         const float4* twg, const float* shift_b, XWork w) {
   WDM_XPASS_PROLOGUE
   for (long long u = (long long)blockIdx.x * C::WARPS + warp; u < nunits; u += wstride) {
     const long long pp = u * C::GROUPS + g;
@@ -867,8 +868,8 @@ __device__ __forceinline__ void adj_kick_points(const float2* v, const float* ph
 
 template <int N>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_adj_kick(float2* __restrict__ lam, const float2* __restrict__ H, float2* __restrict__ Hmu, RowGeom rg,
-              long long hpitch, long long hbstride, const float4* __restrict__ twg, KickArgs a, AdjArgs j, XWork w) {
+k_xw_adj_kick(float2* lam, const float2* H, float2* Hmu, RowGeom rg,
+              long long hpitch, long long hbstride, const float4* twg, KickArgs a, AdjArgs j, XWork w) {
   WDM_XPASS_PROLOGUE
   // With at most WDM_ADJ_PF points per lane the lam and pre rows of the pair
   // fit in registers: row A's are loaded before the potential transform, row
@@ -955,8 +956,8 @@ k_xw_adj_kick(float2* __restrict__ lam, const float2* __restrict__ H, float2* __
 
 template <int N, bool FWD>
 __global__ void __launch_bounds__(XCfg<N>::NT, WDM_X_MINB)
-k_xw_adj_apply(float2* __restrict__ lam, const float2* __restrict__ Hmu, RowGeom rg, long long hpitch,
-               long long hbstride, const float4* __restrict__ twg, AdjArgs j, XWork w) {
+k_xw_adj_apply(float2* lam, const float2* Hmu, RowGeom rg, long long hpitch,
+               long long hbstride, const float4* twg, AdjArgs j, XWork w) {
   WDM_XPASS_PROLOGUE
   for (long long u = (long long)blockIdx.x * C::WARPS + warp; u < nunits; u += wstride) {
     const long long pp = u * C::GROUPS + g;
