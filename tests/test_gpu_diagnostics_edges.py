@@ -94,3 +94,24 @@ def test_device_outputs_of_any_alignment(wdm):
                 buf = torch.zeros(cells + 1, dtype=torch.float32, device="cuda")
                 get(out=buf[off:off + cells].view(n[::-1]))
                 assert np.array_equal(buf[off:off + cells].cpu().numpy().reshape(n[::-1]), host.reshape(n[::-1]))
+
+
+@pytest.mark.parametrize("n,batch", [((8, 8, 8), 1), ((32, 16, 24), 3), ((96, 64, 48), 1), ((128, 128, 96), 1)], ids=str)
+def test_device_inputs_match_host_inputs(wdm, n, batch):
+    # a device psi is stored and summed in one kernel, a host psi copied and then summed: the same bits
+    torch = pytest.importorskip("torch")
+    g = spe.Grid(n, (4.0, 2.0, 3.0))
+    rng = np.random.default_rng(2)
+    shape = ((batch,) if batch > 1 else ()) + n[::-1]
+    psi = (rng.standard_normal(shape) + 1j * rng.standard_normal(shape)).astype(np.complex64)
+    with wdm.SPEContext(n, g.L, poisson_coeff=1.0, batch=batch) as ctx:
+        ctx.set_psi(psi)
+        phi = ctx.get_phi()
+        for off in (0, 1):
+            buf = torch.zeros(psi.size + 1, dtype=torch.complex64, device="cuda")
+            buf[off:off + psi.size] = torch.from_numpy(psi.reshape(-1))
+            torch.cuda.synchronize()
+            ctx.set_psi(buf[off:off + psi.size].view(shape))
+            assert np.array_equal(ctx.get_psi(), psi)
+            # the block sums meet in FP64 atomics: the shift may round the other way in its last place
+            assert np.allclose(ctx.get_phi(), phi, rtol=0, atol=1e-6 * np.abs(phi).max())

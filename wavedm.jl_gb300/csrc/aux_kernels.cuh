@@ -71,7 +71,7 @@ cudaError_t launch_bounded_wait_probe(unsigned long long limit_ns, unsigned long
 cudaError_t launch_sincos_half(const float* h, float* out, long long n, cudaStream_t st);
 // shift[b] = mean over item b of |data|^2 (complex_in) or of data (float), + add
 cudaError_t launch_mean_shift(const void* data, bool complex_in, long long n, int batch, double* sums, float* shift,
-                              double add, cudaStream_t st);
+                              double add, cudaStream_t st, float2* copy = nullptr);
 // fields[b]: the RED_FIELDS of batch item b (partials: nblocks x RED_FIELDS per item)
 cudaError_t launch_reduce(const float2* psi, const float* phi, const RedGeom& g, double* partials, int nblocks,
                           int batch, double* fields, cudaStream_t st);

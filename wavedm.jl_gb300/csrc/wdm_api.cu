@@ -842,17 +842,23 @@ static size_t red_size(const wdm_ctx* c) {  // doubles
   return (size_t)c->d.batch * (((size_t)c->red_blocks + 1) * RED_FIELDS + sizeof(RadiiOut) / sizeof(double));
 }
 
+// A pointer to this device's memory at the alignment that a kernel's access needs
+// (copies take any other pointer that they accept).
+static bool own_memory(const wdm_ctx* c, const void* p, size_t align) {
+  cudaPointerAttributes a{}, own{};
+  if (!p || (uintptr_t)p % align) return false;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&own, c->psi) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == own.device;
+}
+
 // The kernel that makes an output writes it to the caller's buffer itself, if
 // that is this device's memory (256^3: 20 us of copy less); `scratch` and copy_out
 // serve every other pointer.
 static float* output_buffer(const wdm_ctx* c, float* out, int where, float* scratch) {
-  cudaPointerAttributes a{}, own{};
-  if (where != WDM_DEVICE || !out || (uintptr_t)out % 16) return scratch;
-  if (cudaPointerGetAttributes(&a, out) != cudaSuccess || cudaPointerGetAttributes(&own, c->psi) != cudaSuccess) {
-    cudaGetLastError();
-    return scratch;
-  }
-  return a.type == cudaMemoryTypeDevice && a.device == own.device ? out : scratch;
+  return where == WDM_DEVICE && own_memory(c, out, 16) ? out : scratch;
 }
 
 static wdm_status ensure_scratch(wdm_ctx* c) {
@@ -863,8 +869,10 @@ static wdm_status ensure_scratch(wdm_ctx* c) {
 
 // shift[b] = <|psi_b|^2> + mean baryon density: the constant removed from rho
 // before its transform (exact for any value: only k = 0 changes).
-static wdm_status update_shift(wdm_ctx* c) {
-  cudaError_t e = launch_mean_shift(c->psi, true, c->ncell, c->d.batch, c->sums, c->shift, c->rho_b_mean, c->st);
+// from: a new psi on this device, stored as c->psi on the way
+static wdm_status update_shift(wdm_ctx* c, const float2* from = nullptr) {
+  cudaError_t e = launch_mean_shift(from ? from : c->psi, true, c->ncell, c->d.batch, c->sums, c->shift, c->rho_b_mean,
+                                    c->st, from ? c->psi : nullptr);
   if (e != cudaSuccess) return cuda_fail(c, e, "mean shift");
   return WDM_OK;
 }
@@ -1158,10 +1166,16 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
 
 wdm_status wdm_set_psi(wdm_ctx* c, const void* psi, int32_t where) {
   if (!c) return fail(nullptr, WDM_ERR_INVALID, "null context");
-  WDM_TRY(copy_in(c, c->psi, psi, sizeof(float2) * c->ncell * c->d.batch, where));
+  const bool own = where == WDM_DEVICE && own_memory(c, psi, sizeof(float2));
+  if (!own) WDM_TRY(copy_in(c, c->psi, psi, sizeof(float2) * c->ncell * c->d.batch, where));
   WDM_CU(c, cudaMemsetAsync(c->flag, 0, 2 * sizeof(int), c->st));
-  WDM_CU(c, cudaStreamSynchronize(c->st));
-  WDM_TRY(update_shift(c));
+  if (own) {
+    WDM_TRY(update_shift(c, (const float2*)psi));
+    WDM_CU(c, cudaStreamSynchronize(c->st));  // the caller's buffer has been read
+  } else {
+    WDM_CU(c, cudaStreamSynchronize(c->st));
+    WDM_TRY(update_shift(c));
+  }
   c->have_psi = 1;
   c->phi_valid = 0;
   c->psi_y = 0;
