@@ -209,9 +209,9 @@ wdm_status wdm_fft3d(wdm_ctx* ctx, void* data_dev, int32_t dir);
  * share the array: calls whose work overlaps on the GPU race and must be
  * serialised by the caller.
  * It builds its twiddle tables on the device (FP64 sincospi) where wdm_poisson
- * builds them on the host, and it always takes the register-tile line passes
- * and the direct x passes, so its phi agrees with wdm_poisson's to FP32
- * rounding, not bit for bit.
+ * builds them on the host, and it runs Stockham transforms where wdm_poisson runs
+ * two-factor ones, so its phi agrees with wdm_poisson's to FP32 rounding, not bit
+ * for bit.
  * Errors are reported through wdm_last_error(NULL).
  * No counterpart in the reference: it is an addition of this library. */
 wdm_status wdm_poisson_noalloc(const float* rho_dev, float* phi_dev, int32_t nx, int32_t ny, int32_t nz,
@@ -280,16 +280,21 @@ wdm_status wdm_set_profiling(wdm_ctx* ctx, int32_t on);
  * out of a timed run. */
 wdm_status wdm_set_profile_mask(wdm_ctx* ctx, uint64_t mask);
 /* for pass p < WDM_NPASS: launches, summed milliseconds and algorithmic bytes
- * (one read + one write of every operand) of one launch, since profiling on */
+ * (one read + one write of every operand) of one launch, since profiling on.  A
+ * launch that holds several passes (planes that fit one block) counts as one launch
+ * of each and shares its time among them by their bytes. */
 wdm_status wdm_get_profile(wdm_ctx* ctx, int64_t* launches, double* ms, double* bytes_per_launch);
 /* Pass schedule chosen by the autotuner when the context was created, for the
  * passes psi-y, psi-z, H-y, H-z (line passes: impl 0 = TMA-fed persistent
  * pass, 1 = register-tile pass), the kick, the density pass and the density
  * pass with baryons (x passes: impl 0 = rows staged by bulk copies, 1 = rows
- * loaded directly), in that order; ms[2k], ms[2k+1] the best timed
+ * loaded directly; the adjoint's x passes only, the time step has one
+ * implementation of them), in that order; ms[2k], ms[2k+1] the best timed
  * milliseconds of implementations 0 and 1.  The environment variables
  * WDM_SCHEDULE (all seven, comma separated), WDM_LINE_IMPL=tma|tile and
- * WDM_X_IMPL=staged|direct override the choice. */
+ * WDM_X_IMPL=staged|direct override the choice.  WDM_PLANES=off at creation
+ * keeps the y transforms in launches of their own where the x passes would take
+ * them in. */
 wdm_status wdm_get_line_schedule(const wdm_ctx* ctx, int32_t impl[7], double ms[14]);
 /* number of passes and the name of pass p */
 int32_t wdm_num_passes(void);

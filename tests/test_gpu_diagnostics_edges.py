@@ -81,6 +81,26 @@ def test_radii_with_few_weights(wdm, kind):
             _check(ctx, g, n, 1)
 
 
+@pytest.mark.parametrize("power", [-60, -51, 58, 61])
+def test_radii_do_not_depend_on_the_scale(wdm, power):
+    # a power of two scales every weight exactly, whether the FP32 words or FP64 sum it (components
+    # outside 2^-50 .. 2^60); some components are zero
+    n = (48, 32, 64)
+    g = spe.Grid(n, tuple(0.2 * m for m in n))
+    rng = np.random.default_rng(7)
+    psi = (rng.standard_normal(n[::-1]) + 1j * rng.standard_normal(n[::-1])).astype(np.complex64)
+    psi[3, 4, 5] = 0
+    psi[::2, 1, ::3] = psi[::2, 1, ::3].real
+    got = []
+    with wdm.SPEContext(n, g.L, poisson_coeff=0.0) as ctx:
+        for p in (0, power):
+            ctx.set_psi(psi * np.float32(2.0 ** p))
+            d = ctx.diagnostics()
+            got.append([d["argmax"]] + [d[f"radius_{k}0"] for k in range(1, 10)])
+    assert got[0][0] == got[1][0] == np.argmax(np.abs(psi.astype(np.complex128)) ** 2)
+    assert np.allclose(got[1], got[0], rtol=1e-9, atol=0)
+
+
 def test_device_outputs_of_any_alignment(wdm):
     torch = pytest.importorskip("torch")
     n = (32, 16, 24)
