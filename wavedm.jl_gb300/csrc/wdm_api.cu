@@ -842,23 +842,42 @@ static size_t red_size(const wdm_ctx* c) {  // doubles
   return (size_t)c->d.batch * (((size_t)c->red_blocks + 1) * RED_FIELDS + sizeof(RadiiOut) / sizeof(double));
 }
 
-// A pointer to this device's memory at the alignment that a kernel's access needs
-// (copies take any other pointer that they accept).
-static bool own_memory(const wdm_ctx* c, const void* p, size_t align) {
+// cuMemGetAddressRange, resolved from the driver at run time (no -lcuda link).
+static PFN_cuMemGetAddressRange_v3020 address_range() {
+  static PFN_cuMemGetAddressRange_v3020 fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 3020, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(p);
+  }();
+  return fn;
+}
+
+// `bytes` of this device's memory at p, inside one allocation and at the alignment
+// that a kernel's access needs.  Everything else is left to the copies, which
+// check what they are given and refuse a range that is not there.
+static bool own_memory(const wdm_ctx* c, const void* p, size_t bytes, size_t align) {
   cudaPointerAttributes a{}, own{};
   if (!p || (uintptr_t)p % align) return false;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&own, c->psi) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == own.device;
+  if (a.type != cudaMemoryTypeDevice || a.device != own.device) return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const auto range = address_range();
+  if (!range || range(&base, &size, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+  return (uintptr_t)p - (uintptr_t)base + bytes <= size;
 }
 
 // The kernel that makes an output writes it to the caller's buffer itself, if
 // that is this device's memory (256^3: 20 us of copy less); `scratch` and copy_out
 // serve every other pointer.
 static float* output_buffer(const wdm_ctx* c, float* out, int where, float* scratch) {
-  return where == WDM_DEVICE && own_memory(c, out, 16) ? out : scratch;
+  return where == WDM_DEVICE && own_memory(c, out, sizeof(float) * c->ncell * c->d.batch, 16) ? out : scratch;
 }
 
 static wdm_status ensure_scratch(wdm_ctx* c) {
@@ -1166,8 +1185,9 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
 
 wdm_status wdm_set_psi(wdm_ctx* c, const void* psi, int32_t where) {
   if (!c) return fail(nullptr, WDM_ERR_INVALID, "null context");
-  const bool own = where == WDM_DEVICE && own_memory(c, psi, sizeof(float2));
-  if (!own) WDM_TRY(copy_in(c, c->psi, psi, sizeof(float2) * c->ncell * c->d.batch, where));
+  const size_t bytes = sizeof(float2) * c->ncell * c->d.batch;
+  const bool own = where == WDM_DEVICE && own_memory(c, psi, bytes, sizeof(float2));
+  if (!own) WDM_TRY(copy_in(c, c->psi, psi, bytes, where));
   WDM_CU(c, cudaMemsetAsync(c->flag, 0, 2 * sizeof(int), c->st));
   if (own) {
     WDM_TRY(update_shift(c, (const float2*)psi));
