@@ -106,7 +106,6 @@ cudaError_t launch_abs2(const float2* psi, float* out, long long n, cudaStream_t
 // per-cell terms and the precision of the sums unchanged.
 constexpr int RED_THREADS = 128;
 constexpr int RED_CTAS = 5;   // resident blocks an SM
-constexpr int RED_AHEAD = 3;  // steps between a plane's L2 prefetch and its loads (without: 317 -> 297 us)
 // Cells along z of one march: long marches read the planes beside them less often,
 // short ones give every warp of the grid some work.
 static int red_depth(const RedGeom& g, int nblocks) {
@@ -209,10 +208,10 @@ k_reduce(const float2* __restrict__ psi_all, const float* __restrict__ phi_all, 
       ps += nxy;
       fs += nxy;
       if (z + 1 < z1) load(z + 1);
-      if (in && z + RED_AHEAD < z1) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(ps + RED_AHEAD * nxy));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(fs + (RED_AHEAD - 1) * nxy));
-      }
+      // ps and fs are at step z + 1 by now
+      const int ahead = red_ahead_plane(z, z1, g.nz);
+      if (in && ahead >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(ps + (ahead - (z + 1)) * nxy));
+      if (in && z + RED_AHEAD < z1) asm volatile("prefetch.global.L2 [%0];" ::"l"(fs + (RED_AHEAD - 1) * nxy));
       const float mzp = mag(zp);
       const bool inner = xy_inner && z > 0 && z < g.nz - 1;
       const float me = mag(e);

@@ -38,6 +38,14 @@ struct RedGeom {
   int zmid;  // z index of the slice the RED_SW* sums cover
 };
 
+// The plane of psi that step z of a march over the cells z .. z1 - 1 asks L2 for:
+// the one above the cell of step z + RED_AHEAD, which that step loads (k_reduce); -1
+// where no step loads it or the grid of nz planes ends below it.
+constexpr int RED_AHEAD = 3;  // steps between a plane's L2 prefetch and its loads
+__host__ __device__ constexpr int red_ahead_plane(int z, int z1, int nz) {
+  return z + RED_AHEAD < z1 && z + RED_AHEAD + 1 < nz ? z + RED_AHEAD + 1 : -1;
+}
+
 // Lagrangian radii about the density maximum (RED_ARG of `fields`): per squared
 // cell distance key = di^2 + dj^2 + dk^2 the FP64 sum of rho over the cells at
 // that distance (wsum, nkeys words), and what the nine quantiles read of it.
