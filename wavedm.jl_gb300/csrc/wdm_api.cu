@@ -200,6 +200,7 @@ struct wdm_ctx {
   double rho_b_mean = 0.0;          // mean baryon density (static particles)
   int have_psi = 0;
   int phi_valid = 0;
+  int phi_stockham = 0;  // the passes of the adjoint made it (ensure_potential)
   int64_t launch_count = 0;
   // autotuned implementation of each line pass (LP_*) and the candidate timings
   int line_impl[LP_COUNT] = {0, 0, 0, 0, 0, 0, 0};
@@ -662,7 +663,16 @@ static wdm_status density_poisson(wdm_ctx* c, int write_psi, double dt_mask) {
   c->h_y = planes;
   if (!planes) WDM_TRY(potential_rows(c));
   c->phi_valid = 1;
+  c->phi_stockham = c->stockham;
   return WDM_OK;
+}
+
+// The potential of the present psi, from the passes the context is running on: the
+// two families round differently, and what a call returns must not depend on which
+// of them the calls before it ran on.
+static wdm_status ensure_potential(wdm_ctx* c) {
+  if (c->phi_valid && c->phi_stockham == c->stockham) return WDM_OK;
+  return density_poisson(c, 0, 0.0);
 }
 
 static void split_dt(double dt, float* hi, float* lo) {
@@ -1222,7 +1232,7 @@ wdm_status wdm_get_rho(wdm_ctx* c, float* rho, int32_t where) {
 static wdm_status phi_real(wdm_ctx* c, float* out = nullptr) {
   WDM_TRY(ensure_scratch(c));
   float* dst = out ? out : c->scratch_f;
-  if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, 0.0));
+  WDM_TRY(ensure_potential(c));
   // a y-spectral H stays as it is (the next kick and captured graphs start from it)
   float2* H = c->H;
   if (c->h_y) {
@@ -1387,7 +1397,7 @@ static wdm_status step_impl(wdm_ctx* c, int32_t nsteps, double dt, double t0, in
   // kick s runs at time t0 + s dt (the Strang step's closing half kick is kick nsteps)
   if (nsteps == 0) return WDM_OK;
   WDM_TRY(check_tide_rows(c, t0, dt, nsteps + 1, "wdm_step"));
-  if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, dt));
+  WDM_TRY(ensure_potential(c));
   for (int s = 0; s < nsteps; ++s) {
     double kdt;
     if (mode == WDM_STEP_STRANG) kdt = (s == 0) ? 0.5 * dt : dt;  // interior half kicks merged
@@ -1418,7 +1428,7 @@ wdm_status wdm_kick(wdm_ctx* c, double dt, double t) {
                 "wdm_kick: the tidal schedule has several rows but no clock (wdm_set_tidal_clock), so time t "
                 "selects no row");
   WDM_TRY(check_tide_rows(c, t, 0.0, 1, "wdm_kick"));
-  if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, 0.0));
+  WDM_TRY(ensure_potential(c));
   WDM_TRY(kick(c, dt, tide_row(c, t, 0), false));
   return sync_and_check(c);
 }
@@ -1882,7 +1892,6 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
     wdm_ctx* c;
     ~Family() { c->stockham = 0; }
   } family{c};
-  if (c->phi_valid && c->h_y) WDM_TRY(potential_rows(c));
   c->stockham = 1;
   WDM_TRY(ensure_stockham(c));
   const int nck = nsteps / ck + 1;
@@ -1917,7 +1926,7 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
   WDM_CU(c, cudaMemsetAsync(c->adj_acc, 0, sizeof(double) * 2 * B, c->st));
   if (c->d.phase_mode == WDM_PHASE_PRECISE) WDM_TRY(ensure_drift_tables(c, dt));
   if (c->d.absorb_alpha != 0.0) WDM_TRY(ensure_mask_tables(c, dt));
-  if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, dt));
+  WDM_TRY(ensure_potential(c));
   // forward: checkpoints of (s_b, H_b) at b = 0, ck, 2 ck, ...; the states of
   // the last segment go straight into its slots (no recompute needed for it)
   // state s_b of the segment starting at j0: the checkpoint or a slot of its set
@@ -2016,9 +2025,10 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
     }
     if (seg >= 2) WDM_CU(c, cudaEventRecord(c->ev_bwd[seg & 1], c->st));  // its slots may be reused
   }
-  // leave the context at psi_0 with its potential
+  // leave the context at psi_0 with its potential (of this family)
   WDM_TRY(copy_pair(c, c->psi, c->H, c->ck_psi[0], c->ck_H[0]));
   c->phi_valid = 1;
+  c->phi_stockham = 1;
   WDM_TRY(copy_out(c, grad, c->lam, sizeof(float2) * nc, where_g));
   std::vector<double> acc((size_t)2 * B);
   WDM_CU(c, cudaMemcpy(acc.data(), c->adj_acc, sizeof(double) * 2 * B, cudaMemcpyDeviceToHost));
@@ -2079,7 +2089,7 @@ static wdm_status prepare_capture(wdm_ctx* c, double dt) {
   WDM_TRY(need_psi(c));
   if (c->d.phase_mode == WDM_PHASE_PRECISE) WDM_TRY(ensure_drift_tables(c, dt));
   if (c->d.absorb_alpha != 0.0) WDM_TRY(ensure_mask_tables(c, dt));
-  if (!c->phi_valid) WDM_TRY(density_poisson(c, 0, dt));
+  WDM_TRY(ensure_potential(c));
   // the deposit is made once per particle set, here, so a captured sequence
   // holds none
   WDM_TRY(ensure_deposit(c));
