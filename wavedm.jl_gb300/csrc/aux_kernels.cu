@@ -237,7 +237,9 @@ k_reduce(const float2* __restrict__ psi_all, const float* __restrict__ phi_all, 
       const float r0 = a + b;
       const float bb = r0 - a;
       const float r1 = ((a - (r0 - bb)) + (b - bb)) + (ea + eb);
-      const float rs = r0 + r1, rt = r1 - (rs - r0);
+      // beyond FP32 the errors are differences of infinities: rho = r0 alone
+      const bool over = r0 == INFINITY;
+      const float rs = over ? r0 : r0 + r1, rt = over ? 0.f : r1 - (rs - r0);
       if (in && rs >= best_hi) {
         const int i = i0 + (z - z0) * nxy;
         if (rs > best_hi || rt > best_lo || (rt == best_lo && i < best_i)) {
