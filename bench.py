@@ -80,7 +80,10 @@ def ncu_traffic(pass_name, n, workload, sched):
             "phi_y_inv": "h_y"}.get(pass_name)
     if impl is None or impl not in sched:
         return None, "pass not captured"
-    v = cap["passes"].get(f"{pass_name}/{sched[impl]['impl']}")
+    # the step's x passes have one implementation, kept under "staged" (the
+    # schedule's x entries are the adjoint's)
+    name = "staged" if impl.startswith("x_") else sched[impl]["impl"]
+    v = cap["passes"].get(f"{pass_name}/{name}")
     if v is None:
         return None, "pass and implementation not captured"
     same = cap.get("kernel_source_hash") == kernel_source_hash()

@@ -288,8 +288,8 @@ wdm_status wdm_get_profile(wdm_ctx* ctx, int64_t* launches, double* ms, double* 
  * passes psi-y, psi-z, H-y, H-z (line passes: impl 0 = TMA-fed persistent
  * pass, 1 = register-tile pass), the kick, the density pass and the density
  * pass with baryons (x passes: impl 0 = rows staged by bulk copies, 1 = rows
- * loaded directly; the adjoint's x passes only, the time step has one
- * implementation of them), in that order; ms[2k], ms[2k+1] the best timed
+ * loaded directly; the adjoint's x passes, the time step has one
+ * implementation of its own), in that order; ms[2k], ms[2k+1] the best timed
  * milliseconds of implementations 0 and 1.  The environment variables
  * WDM_SCHEDULE (all seven, comma separated), WDM_LINE_IMPL=tma|tile and
  * WDM_X_IMPL=staged|direct override the choice.  WDM_PLANES=off at creation

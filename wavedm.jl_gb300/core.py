@@ -281,7 +281,8 @@ class SPEContext:
                 ("x_rho_b", ("staged", "direct")))
 
     def line_schedule(self):
-        """{pass: dict(impl, ms={impl name: best ms})} as chosen by the autotuner at creation."""
+        """{pass: dict(impl, ms={impl name: best ms})} as chosen by the autotuner at creation
+        (the x entries are the adjoint's passes)."""
         n = len(self.SCHEDULE)
         impl = np.zeros(n, np.int32)
         ms = np.zeros(2 * n, np.float64)

@@ -142,7 +142,7 @@ struct Profiler {
 // 0 is the preferred implementation of each)
 // (LP_X_RHO_B: the density pass with a baryon density to add, which the staged
 // pass prefetches and the direct pass loads after its transform)
-enum { LP_PSI_Y = 0, LP_PSI_Z = 1, LP_H_Y = 2, LP_H_Z = 3, LP_X_KICK = 4, LP_X_RHO = 5, LP_X_RHO_B = 6, LP_COUNT = 7 };
+enum { LP_PSI_Y = 0, LP_PSI_Z = 1, LP_H_Y = 2, LP_H_Z = 3, LP_X_KICK = 4, LP_X_RHO = 5, LP_X_RHO_B = 6, LP_COUNT = 7, LP_LINES = LP_X_KICK };
 
 struct wdm_ctx {
   wdm_desc d{};
@@ -202,11 +202,11 @@ struct wdm_ctx {
   int phi_valid = 0;
   int phi_stockham = 0;  // the passes of the adjoint made it (ensure_potential)
   int64_t launch_count = 0;
-  // autotuned implementation of each line pass (LP_*) and the candidate timings
+  // autotuned implementation of each line pass and of the adjoint's x passes
+  // (LP_*) and the candidate timings
   int line_impl[LP_COUNT] = {0, 0, 0, 0, 0, 0, 0};
-  // the same of the adjoint's Stockham passes, found at the first adjoint
-  int adj_impl[LP_COUNT] = {0, 0, 0, 0, 0, 0, 0};
-  double adj_ms[LP_COUNT][2] = {};
+  // the implementations of the adjoint's line passes, found at the first adjoint
+  int adj_impl[LP_LINES] = {0, 0, 0, 0};
   double line_ms[LP_COUNT][2] = {{-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}, {-1, -1}};
   // adjoint buffers (allocated on first use)
   float2* lam = nullptr;            // adjoint state [batch][ncell]
@@ -510,7 +510,7 @@ static wdm_status ensure_mask_tables(wdm_ctx* c, double dt) {
   return WDM_OK;
 }
 
-// The implementations of the passes the context is running on.
+// The implementations of the line passes the context is running on.
 static int* impls(wdm_ctx* c) { return c->stockham ? c->adj_impl : c->line_impl; }
 static const int* impls(const wdm_ctx* c) { return c->stockham ? c->adj_impl : c->line_impl; }
 
@@ -523,10 +523,10 @@ static RowGeom rows_psi(const wdm_ctx* c) {
   return r;
 }
 
-// The rows of psi for the tuned x pass `kind` (LP_X_KICK, LP_X_RHO or LP_X_RHO_B).
+// The rows of psi for the adjoint's tuned x pass `kind` (LP_X_KICK, LP_X_RHO or LP_X_RHO_B).
 static RowGeom rows_psi(const wdm_ctx* c, int kind) {
   RowGeom r = rows_psi(c);
-  r.impl = impls(c)[kind];
+  r.impl = c->line_impl[kind];
   return r;
 }
 
@@ -953,7 +953,7 @@ wdm_status wdm_destroy(wdm_ctx* c) {
 // Line-pass autotuner
 // --------------------------------------------------------------------------
 // Each line pass (psi and H, along y and z) has two implementations, the
-// TMA-fed persistent pass and the register-tile pass, and the kick and
+// TMA-fed persistent pass and the register-tile pass, and the adjoint's kick and
 // density x passes two, rows staged by bulk copies or loaded directly.  Which
 // is faster depends on the axis length, the width of the rows (the odd
 // nx/2 + 1 of H leaves a mostly empty last 16-line tile), the batch and the
@@ -962,14 +962,15 @@ wdm_status wdm_destroy(wdm_ctx* c) {
 // operator, the kick with a small time step) and keeps the faster, preferring
 // implementation 0 within 3%.  Choices are kept per (device, nx, ny, nz,
 // batch, kernels); WDM_LINE_IMPL=tma|tile and WDM_X_IMPL=staged|direct force
-// them.  The x choices are the adjoint's alone: the row passes of the time
-// step have one implementation.  The adjoint's passes are timed at its first
-// run, on its own buffers.
+// them.  The row passes of the time step have one implementation.  The adjoint's
+// line passes are timed at its first run, on its own buffers.
 using TuneKey = std::tuple<int, int, int, int, int, int>;
 struct TuneVal {
   int impl[LP_COUNT];
   double ms[LP_COUNT][2];
 };
+// passes to time: all of them at creation, the line passes for the adjoint
+static int tuned_passes(const wdm_ctx* c) { return c->stockham ? LP_LINES : LP_COUNT; }
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneVal> g_tune_cache;
 
@@ -977,12 +978,12 @@ static std::map<TuneKey, TuneVal> g_tune_cache;
 static void forced_impls(wdm_ctx* c) {
   if (const char* env = std::getenv("WDM_LINE_IMPL")) {
     if (!std::strcmp(env, "tma") || !std::strcmp(env, "tile"))
-      for (int k = LP_PSI_Y; k <= LP_H_Z; ++k) impls(c)[k] = std::strcmp(env, "tma") ? LINE_IMPL_TILE : LINE_IMPL_TMA;
+      for (int k = 0; k < LP_LINES; ++k) impls(c)[k] = std::strcmp(env, "tma") ? LINE_IMPL_TILE : LINE_IMPL_TMA;
   }
   if (const char* env = std::getenv("WDM_X_IMPL")) {
     if (!std::strcmp(env, "staged") || !std::strcmp(env, "direct"))
       for (int k = LP_X_KICK; k <= LP_X_RHO_B; ++k)
-        impls(c)[k] = std::strcmp(env, "staged") ? X_IMPL_DIRECT : X_IMPL_STAGED;
+        c->line_impl[k] = std::strcmp(env, "staged") ? X_IMPL_DIRECT : X_IMPL_STAGED;
   }
 }
 
@@ -1008,7 +1009,7 @@ static bool schedule_from_env(wdm_ctx* c) {
     if (end == std::string::npos && k + 1 < LP_COUNT) return false;
     pos = end + 1;
   }
-  std::memcpy(impls(c), impl, sizeof(impl));
+  std::copy(impl, impl + tuned_passes(c), impls(c));
   return true;
 }
 
@@ -1024,16 +1025,18 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
   int dev = 0;
   WDM_CU(c, cudaGetDevice(&dev));
   int* impl = impls(c);
-  auto* times = c->stockham ? c->adj_ms : c->line_ms;
+  const int count = tuned_passes(c);
   const TuneKey key{dev, c->d.nx, c->d.ny, c->d.nz, c->d.batch, c->stockham};
   std::lock_guard<std::mutex> lock(g_tune_mu);
   auto hit = g_tune_cache.find(key);
   if (hit != g_tune_cache.end()) {
-    std::memcpy(impl, hit->second.impl, sizeof(hit->second.impl));
-    std::memcpy(times, hit->second.ms, sizeof(hit->second.ms));
+    std::copy(hit->second.impl, hit->second.impl + count, impl);
+    if (!c->stockham) std::memcpy(c->line_ms, hit->second.ms, sizeof(hit->second.ms));
     return WDM_OK;
   }
   const int B = c->d.batch;
+  TuneVal v{};
+  if (!c->twx) WDM_TRY(upload_twiddles(c, &c->twx, c->kx));
   WDM_CU(c, cudaMemsetAsync(c->psi, 0, sizeof(float2) * c->ncell * B, c->st));
   WDM_CU(c, cudaMemsetAsync(c->H, 0, sizeof(float2) * c->nhalf * B, c->st));
   PoissonOp po;
@@ -1053,13 +1056,15 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
       case LP_PSI_Z: return z_poisson(c, c->psi, lines_z(c, c->d.nx, c->d.nx, c->ncell), po);
       case LP_H_Y: return y_lines(c, c->H, lines_y(c, c->nxh, c->hpitch, c->nhalf), false);
       case LP_H_Z: return z_poisson(c, c->H, lines_z(c, c->nxh, c->hpitch, c->nhalf), po);
-      case LP_X_KICK: return x_kick(c, c->psi, ka, true);
-      case LP_X_RHO: return x_rho(c, ra, k);
-      default: {
+      default: {  // the x passes that have a choice are the adjoint's
+        RhoArgs rk = ra;
         // a stand-in baryon density: the zeroed psi buffer, read as floats
-        RhoArgs rb = ra;
-        rb.rho_b = reinterpret_cast<const float*>(c->psi);
-        return x_rho(c, rb, k);
+        if (k == LP_X_RHO_B) rk.rho_b = reinterpret_cast<const float*>(c->psi);
+        const int family = c->stockham;
+        c->stockham = 1;
+        const cudaError_t f = k == LP_X_KICK ? x_kick(c, c->psi, ka, true) : x_rho(c, rk, k);
+        c->stockham = family;
+        return f;
       }
     }
   };
@@ -1067,13 +1072,9 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
   WDM_CU(c, cudaEventCreate(&e0));
   WDM_CU(c, cudaEventCreate(&e1));
   cudaError_t e = cudaSuccess;
-  for (int k = 0; k < LP_COUNT && e == cudaSuccess; ++k) {
+  for (int k = 0; k < count && e == cudaSuccess; ++k) {
     for (int q = 0; q <= 1 && e == cudaSuccess; ++q) {
       impl[k] = q;
-      if (q == 1 && k >= LP_X_KICK && !c->stockham) {  // the two-factor row passes have one implementation
-        times[k][1] = times[k][0];
-        break;
-      }
       double best = 1e30;
       for (int r = 0; r < 4 && e == cudaSuccess; ++r) {  // the first run is a warm-up
         if ((e = cudaEventRecord(e0, c->st)) != cudaSuccess || (e = run(k)) != cudaSuccess ||
@@ -1083,16 +1084,15 @@ static wdm_status tune_passes_timed(wdm_ctx* c) {
         if ((e = cudaEventElapsedTime(&ms, e0, e1)) != cudaSuccess) break;
         if (r > 0 && ms < best) best = ms;
       }
-      times[k][q] = best;
+      v.ms[k][q] = best;
     }
-    impl[k] = times[k][1] < 0.97 * times[k][0] ? 1 : 0;
+    impl[k] = v.ms[k][1] < 0.97 * v.ms[k][0] ? 1 : 0;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (e != cudaSuccess) return cuda_fail(c, e, "line-pass autotuner");
-  TuneVal v;
-  std::memcpy(v.impl, impl, sizeof(v.impl));
-  std::memcpy(v.ms, times, sizeof(v.ms));
+  std::copy(impl, impl + count, v.impl);
+  if (!c->stockham) std::memcpy(c->line_ms, v.ms, sizeof(v.ms));
   g_tune_cache[key] = v;
   return WDM_OK;
 }
@@ -1849,8 +1849,8 @@ static wdm_status forward_boundary_to(wdm_ctx* c, int b, double dt, const float2
   return s;
 }
 
-// The Stockham passes' twiddles and schedule, made at the first adjoint (lam
-// and Hmu, not in use yet, stand in for psi and H in the timings).
+// The Stockham passes' twiddles and the schedule of their line passes, made at the
+// first adjoint (lam and Hmu, not in use yet, stand in for psi and H in the timings).
 static wdm_status ensure_stockham(wdm_ctx* c) {
   if (c->twz) return WDM_OK;
   if (!c->twx) WDM_TRY(upload_twiddles(c, &c->twx, c->kx));
