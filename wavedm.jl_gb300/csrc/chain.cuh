@@ -5,10 +5,12 @@
 // serialisation: a pass's CTAs start, load the twiddle tables (which nothing writes
 // after a context's creation) and set up their barriers before the pass in front has
 // been retired, then wait here for its completion and its memory.  Every CTA
-// waits, so that a pass's completion implies the completion of all before it.  Nothing that another kernel or a copy writes is read before
-// the wait, and none of it through the non-coherent path (no __restrict__ on
-// pointers to it; it measured the same).  The Stockham passes wait before they load
-// their twiddles, which the allocation-free Poisson solve fills on the same stream;
+// waits, so that a pass's completion implies the completion of all before it.
+// Nothing that another kernel or a copy writes is read before the wait, and none of
+// it through the non-coherent path: __restrict__ stands on twiddle tables alone, in
+// the kernels and in the helpers inlined into them (it measured the same).  The
+// Stockham passes wait before they load their twiddles, which the allocation-free
+// Poisson solve fills on the same stream;
 // the adjoint at 128^3, 40 steps, went from 8.5 to 7.3 ms.
 //
 // When the next pass may start:

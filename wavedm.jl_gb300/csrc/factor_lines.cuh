@@ -185,7 +185,7 @@ __device__ __forceinline__ void line_finish(float2* s, float2* base, long long p
 // twiddle table already in shared memory at tw and the exchange buffer s (N
 // LINES entries).
 template <int N, int MODE, class Op>
-__device__ __forceinline__ void line_tile(float2* __restrict__ data, const LineGeom& g, const float4* tw, const Op& op,
+__device__ __forceinline__ void line_tile(float2* data, const LineGeom& g, const float4* tw, const Op& op,
                                           int line0, int b, float2* s, int tid) {
   const int l = tid % LINES, t = tid / LINES;
   const int line = line0 + l;

@@ -488,7 +488,7 @@ __device__ __forceinline__ void rho_lane(At at, float2* base, const RowGeom& rg,
 }
 
 template <int N, bool CEN>
-__device__ __forceinline__ void rho_units(Warp<N>& w, float2* __restrict__ psi, float2* __restrict__ H,
+__device__ __forceinline__ void rho_units(Warp<N>& w, float2* psi, float2* H,
                                           const RowGeom& rg, long long hpitch, long long hbstride, const RhoArgs& a) {
   using R = Rows<N>;
   constexpr int RA = R::RA, RB = R::RB;

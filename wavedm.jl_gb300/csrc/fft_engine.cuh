@@ -390,7 +390,7 @@ template <int N, int T, int R>
 __device__ __forceinline__ int slot_pos(int t, int i, int k) { return t + T * i + k * (N / R); }
 
 // Load `count` entries of a (hi, lo) twiddle table into shared memory.
-__device__ __forceinline__ void load_twiddles(float4* tw_s, const float4* __restrict__ tw_g, int count) {
+__device__ __forceinline__ void load_twiddles(float4* tw_s, const float4* tw_g, int count) {
   for (int i = threadIdx.x; i < count; i += blockDim.x) tw_s[i] = tw_g[i];
 }
 

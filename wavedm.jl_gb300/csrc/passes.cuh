@@ -243,7 +243,7 @@ struct NoOp {
 // with the twiddle tables already in shared memory at tw and the exchange
 // buffer s (N * LPITCH entries).
 template <int N, int MODE, class Op>
-__device__ __forceinline__ void lfft_tile_one(float2* __restrict__ data, const LineGeom& g, const float4* tw,
+__device__ __forceinline__ void lfft_tile_one(float2* data, const LineGeom& g, const float4* tw,
                                               const Op& op, int line0, int b, float2* s, int tid) {
   using P = Plan<N>;
   constexpr int T = P::T;

@@ -313,8 +313,8 @@ struct XWork {
 // Packed potential line of rows (A, B) from their half spectra, loaded at the
 // register slots of radix R: Z[p] = A[p] + i B[p], Z[N-p] = conj A[p] + i conj B[p].
 template <int N, int T, int R>
-__device__ __forceinline__ void load_packed_half(float2* v, const float2* __restrict__ ha,
-                                                 const float2* __restrict__ hb, bool ok, int t) {
+__device__ __forceinline__ void load_packed_half(float2* v, const float2* ha,
+                                                 const float2* hb, bool ok, int t) {
 #pragma unroll
   for (int i = 0; i < N / (R * T); ++i)
 #pragma unroll
@@ -333,8 +333,8 @@ __device__ __forceinline__ void load_packed_half(float2* v, const float2* __rest
 // Hermitian split of the packed forward transform (registers at radix-R slots)
 // into the half spectra of rows A and B (k = 0..N/2), via the group buffer.
 template <int N, int T, int R>
-__device__ __forceinline__ void store_packed_half(const float2* v, float2* buf, float2* __restrict__ ha,
-                                                  float2* __restrict__ hb, bool ok, int t) {
+__device__ __forceinline__ void store_packed_half(const float2* v, float2* buf, float2* ha,
+                                                  float2* hb, bool ok, int t) {
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < N / (R * T); ++i)
@@ -541,7 +541,7 @@ struct XSlice {
 };
 
 template <int N, bool FWD>
-__device__ __forceinline__ void xw_kick_units(const float2* psi_in, float2* psi, const float2* __restrict__ H,
+__device__ __forceinline__ void xw_kick_units(const float2* psi_in, float2* psi, const float2* H,
                                               const RowGeom& rg, long long hpitch, long long hbstride,
                                               const KickArgs& a, const XWork& w, const XSlice& sl) {
   using C = XCfg<N>;
@@ -657,7 +657,7 @@ __device__ __forceinline__ void inv_rho_row(float2* v, const RhoArgs& a, const R
 }
 
 template <int N>
-__device__ __forceinline__ void xw_inv_rho_units(float2* __restrict__ psi, float2* __restrict__ H, const RowGeom& rg,
+__device__ __forceinline__ void xw_inv_rho_units(float2* psi, float2* H, const RowGeom& rg,
                                                  long long hpitch, long long hbstride, const RhoArgs& a,
                                                  const XWork& w, const XSlice& sl) {
   using C = XCfg<N>;
