@@ -22,3 +22,10 @@ def test_only_tables_are_restrict(name, tables):
     found = re.findall(r"([\w ]+)\*\s*__restrict__\s+(\w+)", text)
     assert text.count("__restrict__") == len(found)
     assert [(t, v) for t, v in found if v not in tables or t.split() != ["const", "float4"]] == []
+
+
+def test_tables_go_up_on_the_stream_that_reads_them():
+    """A copy on the default stream is not in front of work on the context's non-blocking stream."""
+    with open(os.path.join(CSRC, "wdm_api.cu"), encoding="utf-8") as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    assert re.findall(r"cudaMemcpy\([^;]*HostToDevice", text) == []

@@ -225,6 +225,7 @@ struct wdm_ctx {
   int rb_ready = 0;
   // diagnostics: radii histogram and its block sums (allocated on first use)
   double* diag_wsum = nullptr;
+  std::vector<std::vector<char>> uploads;  // sources of table copies that may be under way
   long long version = 0;            // bumped by every set_* call that a captured graph bakes in
   struct wdm_group* self_group = nullptr;  // single-member group of wdm_step_graph
   Profiler prof;
@@ -420,22 +421,35 @@ static double kval(int m, int n, double L) {
   return 2.0 * M_PI * s / L;
 }
 
+// Tables go up on the context's stream, in front of the passes that read them (a
+// default-stream copy may still be under way when the call returns, and the
+// context's stream does not wait for it); their sources stay until the stream has
+// been waited for (uploads_done).
+template <class T>
+static wdm_status upload(wdm_ctx* c, T** dst, const std::vector<T>& h) {
+  const char* p = reinterpret_cast<const char*>(h.data());
+  c->uploads.emplace_back(p, p + h.size() * sizeof(T));
+  WDM_TRY(dalloc(c, dst, h.size()));
+  WDM_CU(c, cudaMemcpyAsync(*dst, c->uploads.back().data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, c->st));
+  return WDM_OK;
+}
+static cudaError_t uploads_done(wdm_ctx* c) {
+  const cudaError_t e = cudaStreamSynchronize(c->st);
+  if (e == cudaSuccess) c->uploads.clear();
+  return e;
+}
+
 // The four stage-major (hi, lo) twiddle tables of an axis (TW_TABLES x n).
 static wdm_status upload_twiddles(wdm_ctx* c, float4** dst, const KernelSet* ks) {
-  const int n = ks->n;
-  std::vector<float4> h((size_t)TW_TABLES * n);
+  std::vector<float4> h((size_t)TW_TABLES * ks->n);
   ks->fill_twiddles(h.data());
-  WDM_TRY(dalloc(c, dst, h.size()));
-  WDM_CU(c, cudaMemcpy(*dst, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
-  return WDM_OK;
+  return upload(c, dst, h);
 }
 
 static wdm_status upload_factors(wdm_ctx* c, float4** dst, const FactorSet* fs) {
   std::vector<float4> h((size_t)fs->n);
   fs->fill_twiddles(h.data());
-  WDM_TRY(dalloc(c, dst, h.size()));
-  WDM_CU(c, cudaMemcpy(*dst, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
-  return WDM_OK;
+  return upload(c, dst, h);
 }
 
 static wdm_status upload_k2(wdm_ctx* c, float** dst, int n, double L) {
@@ -444,9 +458,7 @@ static wdm_status upload_k2(wdm_ctx* c, float** dst, int n, double L) {
     const double k = kval(m, n, L);
     h[m] = (float)(k * k);
   }
-  WDM_TRY(dalloc(c, dst, n));
-  WDM_CU(c, cudaMemcpy(*dst, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  return WDM_OK;
+  return upload(c, dst, h);
 }
 
 // Drift factors of the precise form, in FP64 with the phases reduced mod 2 pi
@@ -1185,7 +1197,7 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
   if ((s = tune_passes(c)) != WDM_OK) return bail(s);
   const char* planes_env = std::getenv("WDM_PLANES");  // "off": the separate passes (tests, profiling)
   c->planes = c->fx->plane_ok(d->ny) && !(planes_env && !std::strcmp(planes_env, "off"));
-  if ((e = cudaStreamSynchronize(c->st)) != cudaSuccess) {
+  if ((e = uploads_done(c)) != cudaSuccess) {
     cuda_fail(c, e, "sync");
     return bail(WDM_ERR_CUDA);
   }
@@ -1862,6 +1874,8 @@ static wdm_status ensure_stockham(wdm_ctx* c) {
   c->psi = c->lam;
   c->H = c->Hmu;
   if (s == WDM_OK) s = tune_passes(c);
+  const cudaError_t e = uploads_done(c);
+  if (s == WDM_OK && e != cudaSuccess) s = cuda_fail(c, e, "adjoint tables");
   c->psi = keep_psi;
   c->H = keep_H;
   if (s != WDM_OK && c->twz) {
@@ -1918,8 +1932,8 @@ static wdm_status adjoint_impl(wdm_ctx* c, int nsteps, double dt, int ck, const 
   std::vector<float2*>* set_psi[2] = {&c->slot_psi, &c->slot2_psi};
   std::vector<float2*>* set_H[2] = {&c->slot_H, &c->slot2_H};
   WDM_TRY(copy_in(c, c->rho_t, rho_target, sizeof(float) * nc, where_t));
+  float d6[6];  // until the stream is waited for, below
   if (tidal_dir) {
-    float d6[6];
     for (int q = 0; q < 6; ++q) d6[q] = (float)tidal_dir[q];
     WDM_CU(c, cudaMemcpyAsync(c->D6, d6, sizeof(d6), cudaMemcpyHostToDevice, c->st));
   }
