@@ -71,7 +71,7 @@ struct Launch {
   // grid with fewer units than warps takes smaller CTAs, so that the units
   // spread over the SMs.
   using R = Rows<N>;
-  template <auto K, class... Args>
+  template <auto K, int CTAS, class... Args>
   static cudaError_t rows(const RowGeom& rg, int batch, cudaStream_t st, const Args&... args) {
     XWork w;
     w.pairs_per_item = rg.nrows / 2;
@@ -83,32 +83,32 @@ struct Launch {
     const int sms = sm_count();
     const long long per_sm = (units + sms - 1) / sms;
     const int warps = (int)(per_sm < R::WARPS ? per_sm : R::WARPS);
-    const long long ctas = (units + warps - 1) / warps, cap = (long long)(R::KICK > R::RHO ? R::KICK : R::RHO) * sms;
+    const long long ctas = (units + warps - 1) / warps, cap = (long long)CTAS * sms;
     return launch_chained<K>(dim3((unsigned)(ctas < cap ? ctas : cap)), 32 * warps, R::smem(warps), st, args..., w);
   }
   static cudaError_t fft(float2* data, const RowGeom& rg, const float4* tw, bool inv, float scale, int batch,
                          cudaStream_t st) {
-    return inv ? rows<k_rows_fft<N, true>>(rg, batch, st, data, rg, tw, scale)
-               : rows<k_rows_fft<N, false>>(rg, batch, st, data, rg, tw, scale);
+    return inv ? rows<k_rows_fft<N, true>, R::RHO>(rg, batch, st, data, rg, tw, scale)
+               : rows<k_rows_fft<N, false>, R::RHO>(rg, batch, st, data, rg, tw, scale);
   }
   static cudaError_t rho(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
                          const float4* tw, const RhoArgs& a, int batch, cudaStream_t st) {
-    return a.centre ? rows<k_rows_rho<N, true>>(rg, batch, st, psi, H, rg, hpitch, hbstride, tw, a)
-                    : rows<k_rows_rho<N, false>>(rg, batch, st, psi, H, rg, hpitch, hbstride, tw, a);
+    return a.centre ? rows<k_rows_rho<N, true>, R::RHO>(rg, batch, st, psi, H, rg, hpitch, hbstride, tw, a)
+                    : rows<k_rows_rho<N, false>, R::RHO>(rg, batch, st, psi, H, rg, hpitch, hbstride, tw, a);
   }
   static cudaError_t kick(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg, long long hpitch,
                           long long hbstride, const float4* tw, const KickArgs& a, bool fwd, int batch,
                           cudaStream_t st) {
-    return fwd ? rows<k_rows_kick<N, true>>(rg, batch, st, psi_in, psi, H, rg, hpitch, hbstride, tw, a)
-               : rows<k_rows_kick<N, false>>(rg, batch, st, psi_in, psi, H, rg, hpitch, hbstride, tw, a);
+    return fwd ? rows<k_rows_kick<N, true>, R::KICK>(rg, batch, st, psi_in, psi, H, rg, hpitch, hbstride, tw, a)
+               : rows<k_rows_kick<N, false>, R::KICK>(rg, batch, st, psi_in, psi, H, rg, hpitch, hbstride, tw, a);
   }
   static cudaError_t c2r(const float2* H, float* out, const RowGeom& rg, long long hpitch, long long hbstride,
                          const float4* tw, int batch, cudaStream_t st) {
-    return rows<k_rows_c2r<N>>(rg, batch, st, H, out, rg, hpitch, hbstride, tw);
+    return rows<k_rows_c2r<N>, R::RHO>(rg, batch, st, H, out, rg, hpitch, hbstride, tw);
   }
   static cudaError_t r2c(const float* in, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
                          const float4* tw, const float* shift, int batch, cudaStream_t st) {
-    return rows<k_rows_r2c<N>>(rg, batch, st, in, H, rg, hpitch, hbstride, tw, shift);
+    return rows<k_rows_r2c<N>, R::RHO>(rg, batch, st, in, H, rg, hpitch, hbstride, tw, shift);
   }
   // Plane passes: one CTA per plane, with enough warps for 16 per SM (all that
   // 128 registers a thread allow) over the CTAs that fit; all 16 in one CTA when
