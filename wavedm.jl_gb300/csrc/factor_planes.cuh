@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(32 * PLANE_WARPS, 1) k_plane_rho(PlaneArgs p, 
       });
     }
   }
-  if (CEN && c.n2 == 0) cs.flush(a.centre);
+  if constexpr (CEN) centre_flush(cs, RB, a.centre);
   y_out(c.ny, p.H + c.h0, p.hpitch, c.s, c.hc, c.twy);
 }
 

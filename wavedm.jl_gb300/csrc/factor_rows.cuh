@@ -406,11 +406,13 @@ __device__ __forceinline__ void rows_centre_done(const RhoArgs& a, const RowGeom
     s0b += __shfl_xor_sync(0xffffffffu, s0b, off, RB);
     si += __shfl_xor_sync(0xffffffffu, si, off, RB);
   }
-  if (n2 != 0 || !ok) return;
-  if (cs.item != b) {
-    cs.flush(a.centre);
-    cs.reset(b);
+  if (__any_sync(0xffffffffu, n2 == 0 && ok && cs.item >= 0 && cs.item != b)) {
+    centre_gather(cs, RB, a.centre);
+    if ((threadIdx.x & 31) == 0) cs.flush(a.centre);
+    cs.reset(-1);
   }
+  if (n2 != 0 || !ok) return;
+  if (cs.item < 0) cs.reset(b);
   const int ja = ra % rg.ny, ka = ra / rg.ny, jb = (ra + 1) % rg.ny, kb = (ra + 1) / rg.ny;
   cs.s0 += (double)s0a + (double)s0b;
   cs.si += (double)si;
@@ -519,7 +521,7 @@ __device__ __forceinline__ void rho_units(Warp<N>& w, float2* psi, float2* H,
     packed_out<N>(w, H, hpitch, hbstride);
     __syncwarp();
   }
-  if (CEN && w.n2 == 0) cs.flush(a.centre);
+  if constexpr (CEN) centre_flush(cs, RB, a.centre);
 }
 
 // CEN: also accumulate the density maximum and moments for the tide's frame

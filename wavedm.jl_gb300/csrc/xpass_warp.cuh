@@ -529,7 +529,55 @@ struct CentreSum {
     atomicAdd(reinterpret_cast<double*>(w + 3), sj);
     atomicAdd(reinterpret_cast<double*>(w + 4), sk);
   }
+  // o's share too: added where it is of the same item, else written to its own
+  __device__ __forceinline__ void take(const CentreSum& o, unsigned long long* words) {
+    if (o.item < 0) return;
+    if (item < 0) {
+      *this = o;
+    } else if (o.item != item) {
+      o.flush(words);
+    } else {
+      s0 += o.s0;
+      si += o.si;
+      sj += o.sj;
+      sk += o.sk;
+      key = o.key > key ? o.key : key;
+    }
+  }
 };
+
+// The shares of a warp's lanes 0, stride, 2 stride, ..., brought together on lane 0
+// where they are of one item.  An item's five words are one address each for all SMs,
+// whose atomics queue at about one a nanosecond, so shares are written as seldom as
+// can be: by warp where a unit begins another item, by CTA at the end (a step with a
+// centred tide, against a write per lane: 128 x 96 x 512 273 -> 157 us, eight items of
+// 12 x 384 x 512 2940 -> 750).
+__device__ __forceinline__ void centre_gather(CentreSum& cs, int stride, unsigned long long* words) {
+  const int lane = threadIdx.x & 31;
+  for (int off = 16; off >= stride; off >>= 1) {
+    CentreSum o;
+    o.s0 = __shfl_down_sync(0xffffffffu, cs.s0, off);
+    o.si = __shfl_down_sync(0xffffffffu, cs.si, off);
+    o.sj = __shfl_down_sync(0xffffffffu, cs.sj, off);
+    o.sk = __shfl_down_sync(0xffffffffu, cs.sk, off);
+    o.key = __shfl_down_sync(0xffffffffu, cs.key, off);
+    o.item = __shfl_down_sync(0xffffffffu, cs.item, off);
+    if (lane < off && lane % stride == 0) cs.take(o, words);
+  }
+}
+
+// The same over a CTA of at most CENTRE_WARPS warps, all threads of which get here,
+// and written.
+constexpr int CENTRE_WARPS = 16;
+__device__ __forceinline__ void centre_flush(CentreSum cs, int stride, unsigned long long* words) {
+  __shared__ CentreSum part[CENTRE_WARPS];
+  centre_gather(cs, stride, words);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = cs;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) cs.take(part[w], words);
+  cs.flush(words);
+}
 
 // The slice of an x pass one warp runs: warp units u0, u0 + ustride, ...,
 // with the twiddle tables of the pass (x fwd | x rev) in shared memory at tw
