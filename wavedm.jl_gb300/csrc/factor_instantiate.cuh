@@ -110,12 +110,10 @@ struct Launch {
                          const float4* tw, const float* shift, int batch, cudaStream_t st) {
     return rows<k_rows_r2c<N>, R::RHO>(rg, batch, st, in, H, rg, hpitch, hbstride, tw, shift);
   }
-  // Plane passes: one CTA per plane, with enough warps for 16 per SM (all that
-  // 128 registers a thread allow) over the CTAs that fit; all 16 in one CTA when
-  // there are no more planes than SMs.
-  static bool plane_ok(int ny) {
+  // Plane passes: one CTA per plane.
+  static bool plane_ok(int ny, int planes) {
     if constexpr (Plane<N>::KP == 0) return false;
-    else return plane_ny(ny) && plane_smem<N>(ny) <= PLANE_BYTES;
+    else return plane_ny(ny) && plane_rule(plane_smem<N>(ny), N * ny, planes, sm_count());
   }
   template <auto K, class Args>
   static cudaError_t plane(const PlaneArgs& p, const Args& a, int batch, cudaStream_t st) {
@@ -123,9 +121,7 @@ struct Launch {
     if ((e = prep_once<K>(PLANE_BYTES)) != cudaSuccess) return e;
     const size_t smem = plane_smem<N>(p.rg.ny);
     const int planes = p.rg.nrows / p.rg.ny * batch;
-    const int fit = (int)(228 * 1024 / (smem + 1024));
-    const int warps = planes <= sm_count() || fit <= 1 ? PLANE_WARPS : fit < 8 ? (PLANE_WARPS + fit - 1) / fit : 2;
-    return launch_chained<K>(dim3(planes), 32 * warps, smem, st, p, a);
+    return launch_chained<K>(dim3(planes), 32 * plane_warps(smem, planes, sm_count()), smem, st, p, a);
   }
   static cudaError_t plane_kick(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg,
                                 long long hpitch, long long hbstride, const float4* twx, const float4* twy,

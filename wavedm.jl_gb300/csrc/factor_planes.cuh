@@ -14,7 +14,8 @@
 // gains no more than that of 128^2, and one with longer rows loses (192 x 96 x 48
 // 62 / 66, replayed 43 / 56; 256 x 96 x 256 158 / 169; 64 x 256 x 64 replayed 44 /
 // 48): its three phases run one after another in too few warps.  So rows up to
-// 128 and planes up to PLANE_BYTES (128^2 and its tables) take this path.
+// 128 and planes up to PLANE_BYTES (128^2 and its tables) take this path, where there
+// are enough of them and not too many (plane_rule).
 //
 // The plane is ny rows of RP words.  While it is H, frequency h of row y is at
 // word h; while it is psi, x element (k1, n2), and frequency k1 + RA k2 in its
@@ -53,6 +54,40 @@ WDM_PLANE(128, 9, 148)
 
 constexpr size_t PLANE_BYTES = 156 * 1024;
 constexpr int PLANE_WARPS = 16;  // most warps per CTA (128 registers per thread)
+
+// CTAs per SM that a plane's shared memory leaves room for.
+__host__ __device__ constexpr int plane_fit(size_t smem) {
+  const int fit = (int)(228 * 1024 / (smem + 1024));
+  return fit > 1 ? fit : 1;
+}
+
+// Warps of a plane's CTA: 16 per SM (all that 128 registers a thread allow) over the
+// CTAs that an SM holds at a time, of which there are no more than its share of the
+// planes (by the room alone 256 planes of 48 x 64 got 3 warps each, two CTAs an SM:
+// replayed 52 us a step, now 38, on the separate passes 41).
+__host__ __device__ constexpr int plane_warps(size_t smem, int planes, int sms) {
+  const int fit = plane_fit(smem), share = (planes + sms - 1) / sms;
+  const int ctas = fit < share ? fit : share;
+  return ctas < 8 ? (PLANE_WARPS + ctas - 1) / ctas : 2;
+}
+
+// Whether `planes` planes of `cells` cells are worth a CTA each, against the separate
+// passes (the results are the same bits).  Replayed steps on plane passes / on
+// separate ones, us:
+// - Room for one CTA per SM: only where one wave of them fills the SMs, or there are
+//   so many that the last wave does not count.  Of 128^2: 8 planes 39 / 26, 64 46 /
+//   39, 128 54 / 58, 192 91 / 75, 512 224 / 201, 1024 359 / 389.
+// - For two: not for a few.  96 x 128: 8 planes 34 / 25, 32 36 / 33, 64 41 / 40, 128
+//   56 / 62.
+// - Planes of a few hundred cells: not for thousands, whose CTAs are all overhead.
+//   8^2: 2048 planes 36 / 34, 8192 73 / 42; 24 x 16: 8192 107 / 91; 12 x 64: 92 / 100.
+__host__ __device__ constexpr bool plane_rule(size_t smem, int cells, int planes, int sms) {
+  if (smem > PLANE_BYTES) return false;
+  if (cells <= 512 && planes > 16 * sms) return false;
+  const int fit = plane_fit(smem);
+  if (fit == 1) return (4 * planes >= 3 * sms && planes <= sms) || planes >= 6 * sms;
+  return fit > 2 || 5 * planes >= 2 * sms;
+}
 
 // Rows of the buffer (whole warp units of row pairs) and its bytes with the two
 // twiddle tables.

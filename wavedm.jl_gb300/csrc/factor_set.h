@@ -27,10 +27,10 @@ struct FactorSet {
   cudaError_t (*r2c)(const float* in, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
                      const float4* tw, const float* shift, int batch, cudaStream_t st);
   // plane passes of rows of this length in planes of ny rows (factor_planes.cuh):
-  // whether a plane of them fits a CTA, and the launches (kick: H y-spectral ->
+  // whether so many of them are worth it (plane_rule), and the launches (kick: H y-spectral ->
   // psi x- and y-spectral, or kicked in real space when !fwd; rho: psi x- and
   // y-spectral, or real when !a.write_psi -> H y-spectral)
-  bool (*plane_ok)(int ny);
+  bool (*plane_ok)(int ny, int planes);
   cudaError_t (*plane_kick)(const float2* psi_in, float2* psi, const float2* H, const RowGeom& rg, long long hpitch,
                             long long hbstride, const float4* twx, const float4* twy, const KickArgs& a, bool fwd,
                             int batch, cudaStream_t st);

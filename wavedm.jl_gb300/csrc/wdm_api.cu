@@ -1196,7 +1196,7 @@ wdm_status wdm_create(const wdm_desc* d, wdm_ctx** out) {
   }
   if ((s = tune_passes(c)) != WDM_OK) return bail(s);
   const char* planes_env = std::getenv("WDM_PLANES");  // "off": the separate passes (tests, profiling)
-  c->planes = c->fx->plane_ok(d->ny) && !(planes_env && !std::strcmp(planes_env, "off"));
+  c->planes = c->fx->plane_ok(d->ny, d->nz * d->batch) && !(planes_env && !std::strcmp(planes_env, "off"));
   // the default stream too: a caller's inputs that were queued there before this call
   // are complete after it, and the context's stream does not wait for them
   if ((e = uploads_done(c)) != cudaSuccess || (e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) {
