@@ -20,16 +20,21 @@
 //   373 -> 422 (without overlap at all 1302 and 391).
 // - At the start in grids of at most CHAIN_SMALL threads, which leave most SMs empty
 //   in any case: 64^3 23.3 -> 21.1 us a step (without overlap 31.9), 48^3 23.3 -> 20.7.
+//   Row passes, whose CTAs stay longest, at most CHAIN_SMALL_ROWS: replayed 192 x 32 x
+//   32 (8192 threads) 36.2 -> 29.1, 192 x 48 x 8 28.6 -> 27.2, 256 x 8 x 48 33.9 ->
+//   27.8; but 128 x 256 x 16 (16384) 34.8 -> 37.6, 192 x 96 x 48 (18432) 42.6 -> 49.5.
 #pragma once
 
 namespace wdm {
 
 constexpr unsigned CHAIN_SMALL = 32768;
+constexpr unsigned CHAIN_SMALL_ROWS = 8192;
 
-template <bool TRIGGER>
+// MOST: the most threads of a grid that lets the next pass start (0: none does).
+template <unsigned MOST>
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  if (TRIGGER && gridDim.x * gridDim.y * blockDim.x <= CHAIN_SMALL)
+  if (MOST && gridDim.x * gridDim.y * blockDim.x <= MOST)
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 

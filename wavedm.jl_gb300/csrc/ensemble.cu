@@ -239,7 +239,7 @@ size_t smem_for_axis(int n, int kind) {  // kind 0: x pass, else lines
 
 __global__ void k_tide_frame(const unsigned long long* words, KickArgs a, int mode, int nx, int ny,
                              int batch, float* frame) {
-  chain_wait<true>();
+  chain_wait<CHAIN_SMALL>();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += gridDim.x * blockDim.x) {
     float T6[6];
     for (int q = 0; q < 6; ++q) T6[q] = a.T6b ? a.T6b[6 * b + q] : a.T6[q];

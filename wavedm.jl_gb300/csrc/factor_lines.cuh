@@ -208,7 +208,7 @@ k_line_tile(float2* data, LineGeom g, const float4* __restrict__ twg, Op op) {
   float4* tw = reinterpret_cast<float4*>(smem);
   load_twiddles(tw, twg, N);
   if (MODE == 1) __syncthreads();  // else visible after the tile's first barrier
-  chain_wait<true>();
+  chain_wait<CHAIN_SMALL>();
   line_tile<N, MODE, Op>(data, g, tw, op, blockIdx.x * LINES, blockIdx.y, smem + 2 * N, threadIdx.x);
 }
 
@@ -305,7 +305,7 @@ k_line_tma(float2* data, const __grid_constant__ CUtensorMap map, const __grid_c
     mbar_fence_init();
   }
   load_twiddles(tw, twg, N);
-  chain_wait<false>();
+  chain_wait<0>();
   if constexpr (STAGED)
     for (int i = tid; i < N; i += blockDim.x) optab[i] = op.entry(i);
   __syncthreads();

@@ -238,7 +238,7 @@ struct PlaneCta {
     hc = Columns{N / 2 + 1, 0, 0, RP};
     pc = Columns{N, R::RA, KP, RP};
     __syncthreads();
-    chain_wait<true>();
+    chain_wait<CHAIN_SMALL>();
   }
   __device__ __forceinline__ int units() const { return (ny / 2 + R::PW - 1) / R::PW; }
   __device__ __forceinline__ float2* row(int y) const { return s + y * RP; }

@@ -83,7 +83,7 @@ struct Warp {
     float4* t = reinterpret_cast<float4*>(smem);
     load_twiddles(t, twg, N);
     __syncthreads();
-    chain_wait<false>();
+    chain_wait<CHAIN_SMALL_ROWS>();
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
     set(t, smem + 2 * N + (size_t)warp * R::WORDS, w, blockIdx.x * warps + warp, gridDim.x * warps);
   }

@@ -285,7 +285,7 @@ k_lfft_tile(float2* data, LineGeom g, const float4* twg, Op op) {
   extern __shared__ float2 smem[];
   float4* tw = reinterpret_cast<float4*>(smem);  // line fwd [| line rev] tables
   float2* s = smem + 2 * NTAB * N;
-  chain_wait<false>();
+  chain_wait<0>();
   load_twiddles(tw, twg + TW_LINE_FWD * N, NTAB * N);
   lfft_tile_one<N, MODE, Op>(data, g, tw, op, blockIdx.x * LINES, blockIdx.y, s, threadIdx.x);
 }
@@ -389,7 +389,7 @@ k_lfft_tma(float2* data, const __grid_constant__ CUtensorMap map, const __grid_c
     mbar_init(&bar[1], 1);
     mbar_fence_init();
   }
-  chain_wait<false>();
+  chain_wait<0>();
   load_twiddles(tw, twg + TW_LINE_FWD * N, NTAB * N);
   if constexpr (MODE == 2 && Op::TABLE)
     for (int i = tid; i < N; i += blockDim.x) optab[i] = op.table_entry(i);

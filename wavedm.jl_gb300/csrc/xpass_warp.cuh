@@ -375,7 +375,7 @@ __device__ __forceinline__ void store_packed_half(const float2* v, float2* buf, 
   (void)R1;                                                                         \
   (void)RS;                                                                         \
   extern __shared__ float2 smem[];                                                  \
-  chain_wait<false>();                                                              \
+  chain_wait<0>();                                                              \
   WDM_XPASS_TWIDDLES                                                                \
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;                       \
   const int g = lane / T, t = lane % T;                                             \
