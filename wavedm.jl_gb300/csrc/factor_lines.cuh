@@ -229,7 +229,11 @@ __host__ __device__ constexpr size_t line_tile_smem() {
 // Shared memory of a CTA: the tile slots, the twiddle table, two mbarriers and
 // (MODE 2) the operator's table along the lines.  CTAs per SM follow from it
 // and from the registers; a CTA has two tile slots where that costs no CTA,
-// else one (384^3: four CTAs of one slot, z pass 234 us; three CTAs, 243 us).
+// else one (384^3: four CTAs of one slot, z pass 234 us; three CTAs, 243 us).  The
+// plain passes of 384 and 512 points have two slots at half the CTAs all the same:
+// bound by memory, they gain more from a copy that is always under way (psi y and H y
+// passes, forward and inverse, 384^3: 160, 159, 97, 89 -> 158, 156, 93, 86 us; 512 x
+// 512 x 256: 179, 188, 111, 115 -> 177, 184, 106, 104; 256^3: 51, 44, 31, 26 either way).
 // The drift's table of four words per point is staged where that costs at
 // most one CTA in seven (384: one in four, z pass 234 us without it, 243 us with
 // it; 24 halos of 96^3: two in fifteen, 90 us without it, 81 us with it).
@@ -242,19 +246,20 @@ __host__ __device__ constexpr int line_tma_ctas_of(int slots, size_t entry) {
   const int s = (int)((228u * 1024u) / (line_tma_smem_of<N>(slots, entry) + 1024u));
   return s < 1 ? 1 : s < line_ctas<N>() ? s : line_ctas<N>();
 }
-template <int N>
+template <int N, int MODE>
 __host__ __device__ constexpr int line_tma_slots() {
+  if (MODE != 2 && N >= 384) return 2;
   return line_tma_ctas_of<N>(2, sizeof(float)) == line_tma_ctas_of<N>(1, sizeof(float)) ? 2 : 1;
 }
 template <int N, int MODE, class Op>
 __host__ __device__ constexpr bool line_tma_staged() {
   return MODE == 2 && (sizeof(typename Op::Entry) == sizeof(float) ||
-                       7 * line_tma_ctas_of<N>(line_tma_slots<N>(), sizeof(typename Op::Entry)) >=
-                           6 * line_tma_ctas_of<N>(line_tma_slots<N>(), sizeof(float)));
+                       7 * line_tma_ctas_of<N>(line_tma_slots<N, MODE>(), sizeof(typename Op::Entry)) >=
+                           6 * line_tma_ctas_of<N>(line_tma_slots<N, MODE>(), sizeof(float)));
 }
 template <int N, int MODE, class Op>
 __host__ __device__ constexpr size_t line_tma_smem() {
-  return line_tma_smem_of<N>(line_tma_slots<N>(), line_tma_staged<N, MODE, Op>() ? sizeof(typename Op::Entry) : 0);
+  return line_tma_smem_of<N>(line_tma_slots<N, MODE>(), line_tma_staged<N, MODE, Op>() ? sizeof(typename Op::Entry) : 0);
 }
 
 // Ask L2 for a full tile's boxes (ltma_issue's coordinates; edge tiles are small).
@@ -274,11 +279,11 @@ __device__ __forceinline__ void line_tma_prefetch(const CUtensorMap* map, const 
 }
 
 template <int N, int MODE, class Op, bool LATE>
-__global__ void __launch_bounds__(line_threads<N>(), (line_tma_ctas_of<N>(line_tma_slots<N>(), sizeof(float))))
+__global__ void __launch_bounds__(line_threads<N>(), (line_tma_ctas_of<N>(line_tma_slots<N, MODE>(), sizeof(float))))
 k_line_tma(float2* data, const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap emap,
            LineGeom g, const float4* __restrict__ twg, Op op, int batch) {
   using TT = TmaTile<N>;
-  constexpr int SLOTS = line_tma_slots<N>();
+  constexpr int SLOTS = line_tma_slots<N, MODE>();
   constexpr bool STAGED = line_tma_staged<N, MODE, Op>();
   extern __shared__ __align__(1024) unsigned char lsm[];
   float2* slots = reinterpret_cast<float2*>(lsm);
