@@ -142,6 +142,15 @@ struct Launch {
       return a.centre ? plane<k_plane_rho<N, true>>(p, a, batch, st) : plane<k_plane_rho<N, false>>(p, a, batch, st);
     }
   }
+  static cudaError_t plane_c2r(const float2* H, float* out, const RowGeom& rg, long long hpitch, long long hbstride,
+                               const float4* twx, const float4* twy, int batch, cudaStream_t st) {
+    if constexpr (Plane<N>::KP == 0) {
+      return cudaErrorInvalidValue;
+    } else {
+      const PlaneArgs p{nullptr, nullptr, const_cast<float2*>(H), rg, hpitch, hbstride, twx, twy};
+      return plane<k_plane_c2r<N>>(p, out, batch, st);
+    }
+  }
   static void fill_twiddles(float4* out) {
     fill_factor_twiddles<N>(out, [](long long m) {
       const double a = -2.0 * 3.14159265358979323846 * (double)m / (double)N;
@@ -150,7 +159,7 @@ struct Launch {
   }
   static const FactorSet* set() {
     static const FactorSet fs = {N,    &line, &line_drift, &line_poisson, &fft,       &rho,          &kick,
-                                 &c2r, &r2c,  &plane_ok,   &plane_kick,   &plane_rho, &fill_twiddles};
+                                 &c2r, &r2c,  &plane_ok,   &plane_kick,   &plane_rho, &plane_c2r,    &fill_twiddles};
     return &fs;
   }
 };

@@ -244,32 +244,63 @@ struct PlaneCta {
   __device__ __forceinline__ float2* row(int y) const { return s + y * RP; }
 };
 
+// The packed lines of unit u replace the half spectra they come from, once all of the
+// unit's are in registers.
+template <int N>
+__device__ __forceinline__ void plane_packed_in(const PlaneCta<N>& c, int u) {
+  using R = Rows<N>;
+  constexpr int RA = R::RA, RB = R::RB, PW = R::PW, KP = Plane<N>::KP, ROUNDS = (PW * RA + 31) / 32;
+  float2 v[ROUNDS][RB];
+#pragma unroll
+  for (int i = 0; i < ROUNDS; ++i) {
+    const int q = c.lane + 32 * i, y = 2 * (u * PW + q / RA);
+    pack_half<N>(v[i], c.row(y), c.row(y + 1), q < PW * RA, q % RA);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < ROUNDS; ++i) {
+    const int q = c.lane + 32 * i;
+    if (q < PW * RA) b_inverse<N>(c.twx, v[i], c.row(2 * (u * PW + q / RA)) + (q % RA) * KP, q % RA);
+  }
+}
+
+// Phi in real space (rows of `out` as those of psi) from a y-spectral H, which stays.
+template <int N>
+__global__ void __launch_bounds__(32 * PLANE_WARPS, 1) k_plane_c2r(PlaneArgs p, float* out) {
+  using R = Rows<N>;
+  constexpr int RA = R::RA, RB = R::RB, PW = R::PW, KP = Plane<N>::KP;
+  extern __shared__ __align__(16) float2 smem[];
+  PlaneCta<N> c(smem, p);
+  y_in(c.ny, p.H + c.h0, p.hpitch, c.s, c.hc, c.twy);
+  for (int u = c.warp; u < c.units(); u += blockDim.x >> 5) {
+    plane_packed_in(c, u);
+    __syncwarp();
+    const int y = 2 * (u * PW + c.pr);
+    float2 z[RA];
+#pragma unroll
+    for (int k1 = 0; k1 < RA; ++k1) z[k1] = c.row(y)[k1 * KP + c.n2];
+    dftR<RA, true>(z);
+    float* oa = out + c.psi0 + (long long)y * p.rg.pitch + c.n2;
+    if (y < c.ny)
+#pragma unroll
+      for (int n1 = 0; n1 < RA; ++n1) {
+        oa[RB * n1] = z[n1].x;
+        oa[p.rg.pitch + RB * n1] = z[n1].y;
+      }
+  }
+}
+
 template <int N, bool FWD>
 __global__ void __launch_bounds__(32 * PLANE_WARPS, 1) k_plane_kick(PlaneArgs p, KickArgs a) {
   using R = Rows<N>;
-  constexpr int RA = R::RA, RB = R::RB, PW = R::PW, KP = Plane<N>::KP, ROUNDS = (PW * RA + 31) / 32;
+  constexpr int RA = R::RA, RB = R::RB, PW = R::PW, KP = Plane<N>::KP;
   extern __shared__ __align__(16) float2 smem[];
   PlaneCta<N> c(smem, p);
   y_in(c.ny, p.H + c.h0, p.hpitch, c.s, c.hc, c.twy);
   float T6[10];
   kick_tidal<N>(T6, a, p.rg, c.b);
   for (int u = c.warp; u < c.units(); u += blockDim.x >> 5) {
-    {
-      // the packed lines replace the half spectra they come from, once all of
-      // the unit's are in registers
-      float2 v[ROUNDS][RB];
-#pragma unroll
-      for (int i = 0; i < ROUNDS; ++i) {
-        const int q = c.lane + 32 * i, y = 2 * (u * PW + q / RA);
-        pack_half<N>(v[i], c.row(y), c.row(y + 1), q < PW * RA, q % RA);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < ROUNDS; ++i) {
-        const int q = c.lane + 32 * i;
-        if (q < PW * RA) b_inverse<N>(c.twx, v[i], c.row(2 * (u * PW + q / RA)) + (q % RA) * KP, q % RA);
-      }
-    }
+    plane_packed_in(c, u);
     const int y = 2 * (u * PW + c.pr);
     const bool ok = y < c.ny;
     const int ra = c.z * c.ny + (ok ? y : 0);

@@ -36,6 +36,9 @@ struct FactorSet {
                             int batch, cudaStream_t st);
   cudaError_t (*plane_rho)(float2* psi, float2* H, const RowGeom& rg, long long hpitch, long long hbstride,
                            const float4* twx, const float4* twy, const RhoArgs& a, int batch, cudaStream_t st);
+  // H y-spectral -> Phi in real space (H stays)
+  cudaError_t (*plane_c2r)(const float2* H, float* out, const RowGeom& rg, long long hpitch, long long hbstride,
+                           const float4* twx, const float4* twy, int batch, cudaStream_t st);
   // host: fill the n-entry twiddle table of this axis length
   void (*fill_twiddles)(float4* out);
 };

@@ -1248,19 +1248,15 @@ static wdm_status phi_real(wdm_ctx* c, float* out = nullptr) {
   float* dst = out ? out : c->scratch_f;
   WDM_TRY(ensure_potential(c));
   // a y-spectral H stays as it is (the next kick and captured graphs start from it)
-  float2* H = c->H;
-  if (c->h_y) {
-    WDM_CU(c, cudaMemcpyAsync(c->scratch_h, c->H, sizeof(float2) * c->nhalf * c->d.batch, cudaMemcpyDeviceToDevice, c->st));
-    c->H = c->scratch_h;
-    wdm_status s = potential_rows(c);
-    c->H = H;
-    c->h_y = 1;
-    WDM_TRY(s);
-    H = c->scratch_h;
-  }
-  cudaError_t e = run_pass(c, P_PHI_OUT, [&] {
-    return c->fx->c2r(H, dst, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
-  });
+  cudaError_t e;
+  if (c->h_y)
+    e = run_passes(c, {P_H_Y_INV, P_PHI_OUT}, [&] {
+      return c->fx->plane_c2r(c->H, dst, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->fty, c->d.batch, c->st);
+    });
+  else
+    e = run_pass(c, P_PHI_OUT, [&] {
+      return c->fx->c2r(c->H, dst, rows_psi(c), c->hpitch, c->nhalf, c->ftx, c->d.batch, c->st);
+    });
   if (e != cudaSuccess) return cuda_fail(c, e, "x_c2r");
   return WDM_OK;
 }
