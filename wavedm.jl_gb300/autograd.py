@@ -20,7 +20,10 @@ class EvolveLoss(torch.autograd.Function):
         spe_ctx.set_psi(psi0.detach().contiguous())
         spe_ctx.set_tidal([float(amp) * D])
         if not (ctx_.needs_input_grad[0] or ctx_.needs_input_grad[1]):
-            # no gradient wanted: the forward run alone (the adjoint costs ~2.5 of them)
+            # no gradient wanted: the forward run alone, on the time step's transforms (the
+            # adjoint, on its own, costs ~3.3 of them); the loss is the one that comes with
+            # gradients to the rounding of an FP32 run (40 steps of 32^3: 2e-7 apart, their
+            # errors 8e-8 and 1.4e-7; 128^3: 3e-8)
             spe_ctx.step(nsteps, dt)
             rho = torch.empty(psi0.shape, dtype=torch.float32, device=psi0.device)
             spe_ctx.get_rho(rho)

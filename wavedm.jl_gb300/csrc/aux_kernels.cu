@@ -100,10 +100,11 @@ cudaError_t launch_abs2(const float2* psi, float* out, long long n, cudaStream_t
 // below and the cell above it in registers: a cell's psi and |psi| are loaded and
 // formed once as the cell above, its x neighbours come from the neighbouring
 // lanes (the outer lanes load theirs), its y neighbours from memory (L1: the next
-// warps' rows).  A step's loads are issued one step ahead, behind an L2 prefetch.  That is four square roots per cell instead of seven.  Bound by
-// instruction issue (300 a cell, 63% of the slots: the per-cell terms, four IEEE
-// roots, a division, eleven compensated sums); 256^3 350 -> 210 us, with the
-// per-cell terms and the precision of the sums unchanged.
+// warps' rows).  A step's loads are issued one step ahead, behind an L2 prefetch.
+// That is four square roots per cell instead of seven.  Bound by instruction issue
+// (300 a cell, 63% of the slots: the per-cell terms, four IEEE roots, a division,
+// eleven compensated sums); 256^3 350 -> 210 us, with the per-cell terms and the
+// precision of the sums unchanged.
 constexpr int RED_THREADS = 128;
 constexpr int RED_CTAS = 5;   // resident blocks an SM
 // Cells along z of one march: long marches read the planes beside them less often,
@@ -116,10 +117,11 @@ static int red_depth(const RedGeom& g, int nblocks) {
 }
 
 // Two running sums side by side as unevaluated float pairs hi + lo (Knuth's
-// two-sum moves every rounding error of hi into lo).  A thread adds a few
-// hundred terms, so hi + lo carries each sum to about 2^-44 relative: FP64
-// accuracy for the totals without FP64 arithmetic per cell, which this GPU
-// runs at a small fraction of its FP32 rate.
+// two-sum moves every rounding error of hi into lo).  What is lost are the roundings of
+// lo itself: with the n of 1,400 terms that a thread adds at most (512^3 over 760 blocks
+// of 128) about 2^-50 n / 2 = 2^-40 of its sum as roundings fall, n^2 / 3 2^-48 = 2^-28
+// at the worst, and less of the total of all threads.  FP64 arithmetic per cell runs at
+// a small fraction of the FP32 rate on this GPU.
 struct FAcc2 {
   float2 hi = {0.f, 0.f}, lo = {0.f, 0.f};
   __device__ __forceinline__ void add(float u, float v) {

@@ -20,6 +20,9 @@
 //   373 -> 422 (without overlap at all 1302 and 391).
 // - At the start in grids of at most CHAIN_SMALL threads, which leave most SMs empty
 //   in any case: 64^3 23.3 -> 21.1 us a step (without overlap 31.9), 48^3 23.3 -> 20.7.
+//   The line, against a quarter and four times of it (8192 / 32768 / 131072), us a
+//   step: 32^3 15.4 / 14.4 / 14.4, 64^3 23.1 / 20.8 / 20.8, two of 64^3 24.2 / 24.2 /
+//   24.7, 96^3 38.8 / 38.5 / 44.1, 64 x 96 x 64 26.3 / 26.0 / 25.4.
 //   Row passes, whose CTAs stay longest, at most CHAIN_SMALL_ROWS: replayed 192 x 32 x
 //   32 (8192 threads) 36.2 -> 29.1, 192 x 48 x 8 28.6 -> 27.2, 256 x 8 x 48 33.9 ->
 //   27.8; but 128 x 256 x 16 (16384) 34.8 -> 37.6, 192 x 96 x 48 (18432) 42.6 -> 49.5.

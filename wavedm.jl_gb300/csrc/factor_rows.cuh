@@ -36,7 +36,11 @@ namespace fx {
 // 384^3 12 warps of 168 registers 232 / 223, 16 of 128 279 / 318; 256^3 16 of 128
 // 68 / 68, 20 of 96 83 / 94; 512^3 8 of 255 603 / 518, 12 of 168 625 / 571; 96
 // halos of 64^3 20 of 96 102 / 104, 32 of 64 95 / 113; 24 of 96^3 16 of 128 101 /
-// 93, 20 of 96 94 / 90.
+// 93, 20 of 96 94 / 90.  65536 rows: of 192 points 12 of 168 64 / 62, 8 of 255 69 / 70,
+// 16 of 128 75 / 72; of 128 16 of 128 37 / 31, 12 of 168 41 / 35, 20 of 96 43 / 36; of
+// 48 20 of 96 20.5 / 19.1, 28 of 72 20.6 / 20.4; of 32 32 of 64 14.4 / 14.3, 20 of 96
+// 15.1 / 14.4, 36 of 56 15.1 / 15.9; of 24 12.9 / 12.3, 20 14.4 / 14.1, 48 14.4 / 16.4;
+// of 16, 12 and 8 32 and 20 warps within 3%, more warps slower.
 template <int N>
 struct Rows;
 #define WDM_ROWS(N_, KP_, RP_, WARPS_, KICK_, RHO_)                                      \

@@ -275,9 +275,7 @@ __device__ __forceinline__ void lfft_tile_one(float2* data, const LineGeom& g, c
 
 // One tile of LINES lines per CTA (lfft_tile_one); the hardware overlaps one
 // resident CTA's loads with another's arithmetic.  This is the line pass where
-// the array has no tensor-map view (or the autotuner prefers it); the
-// persistent cp.async pipeline above is kept behind WDM_LINE_PIPELINE for
-// tuning.
+// the array has no tensor-map view (or the autotuner prefers it).
 template <int N, int MODE, class Op>
 __global__ void __launch_bounds__(threads_for<N>(), min_blocks<N>())
 k_lfft_tile(float2* data, LineGeom g, const float4* twg, Op op) {

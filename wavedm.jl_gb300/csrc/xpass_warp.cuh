@@ -550,8 +550,8 @@ struct CentreSum {
 // where they are of one item.  An item's five words are one address each for all SMs,
 // whose atomics queue at about one a nanosecond, so shares are written as seldom as
 // can be: by warp where a unit begins another item, by CTA at the end (a step with a
-// centred tide, against a write per lane: 128 x 96 x 512 273 -> 157 us, eight items of
-// 12 x 384 x 512 2940 -> 750).
+// centred tide, against a write per lane: 128 x 96 x 512 on plane passes 275 -> 199 us,
+// eight items of 12 x 384 x 512 3243 -> 747).
 __device__ __forceinline__ void centre_gather(CentreSum& cs, int stride, unsigned long long* words) {
   const int lane = threadIdx.x & 31;
   for (int off = 16; off >= stride; off >>= 1) {
